@@ -38,11 +38,16 @@ _lib = None
 REFERENCE_DIR = os.environ.get("POLYMER_REFERENCE", "/root/reference")
 
 
+def reference_present() -> bool:
+    """Whether REFERENCE_DIR holds the reference's sources (the folder may exist and be empty)."""
+    return os.path.isfile(os.path.join(REFERENCE_DIR, "numa-PageRank.C"))
+
+
 def build() -> None:
     """Compile the C restatement (and, when the reference sources are
     present, the reference binaries) with make."""
     targets = ["oracle"]
-    if os.path.isdir(REFERENCE_DIR):
+    if reference_present():
         targets.append("ref")
     subprocess.run(["make", "-s", "-C", HERE, "REF=" + REFERENCE_DIR] + targets, check=True)
 
