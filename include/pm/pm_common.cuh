@@ -47,6 +47,22 @@ PM_CXX_API long long launches(bool reset);
     PM_CUDA(cudaGetLastError());                                             \
   } while (0)
 
+// The same for a cooperative launch (grid-wide barriers): the arguments are
+// converted to the kernel's parameter types.
+template <class T>
+struct Same {
+  using type = T;
+};
+template <class... P>
+inline void launch_coop(void (*kernel)(P...), int grid, int block, cudaStream_t stream,
+                        typename Same<P>::type... args) {
+  void *ptrs[] = {(void *)&args...};
+  PM_CUDA(cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(block), ptrs, 0, stream));
+  count_launch();
+}
+#define PM_LAUNCH_COOP(kernel, grid, block, stream, ...) \
+  ::pm::launch_coop(kernel, (grid), (block), (stream), __VA_ARGS__)
+
 constexpr int kWarp = 32;
 constexpr int kDevBFInf = 1073741823;  // INT_MAX / 2
 

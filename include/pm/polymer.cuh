@@ -1368,6 +1368,7 @@ struct Profiler {
   struct Rec {
     std::string tag;
     cudaEvent_t a, b;
+    int passes;  // application passes the bracket covers
   };
   struct Total {
     std::string tag;
@@ -1396,9 +1397,9 @@ struct Profiler {
     else
       PM_CUDA(cudaEventRecord(e, s));
   }
-  void begin(const char *tag, cudaStream_t s) {
+  void begin(const char *tag, cudaStream_t s, int passes = 1) {
     if (!enabled) return;
-    Rec r{tag, take(), take()};
+    Rec r{tag, take(), take(), passes};
     record(r.a, s);
     (capturing ? captured : recs).push_back(r);
   }
@@ -1413,10 +1414,10 @@ struct Profiler {
     for (auto &t : totals)
       if (t.tag == r.tag) {
         t.ms += ms;
-        t.passes++;
+        t.passes += r.passes;
         return;
       }
-    totals.push_back(Total{r.tag, (double)ms, 1});
+    totals.push_back(Total{r.tag, (double)ms, r.passes});
   }
   // The stream has drained: fold the pending brackets.
   void fold() {

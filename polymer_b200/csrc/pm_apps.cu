@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "pm_bp.cuh"
 #include "pm_graph.cuh"
 
 namespace pm {
@@ -899,14 +900,6 @@ void run_spmv(pm_graph *g, const T *d_x0, int iters, T *d_y, double *d_norm) {
 // the frontier: the pull reduces k_d and commit() applies it, in logs.
 // Messages are normalised to sum 1 (see pm_bp in the header).
 // ===========================================================================
-template <class T> struct Vec2;
-template <> struct Vec2<float> { using type = float2; };
-template <> struct Vec2<double> { using type = double2; };
-__device__ __forceinline__ float bp_exp(float x) { return expf(x); }
-__device__ __forceinline__ double bp_exp(double x) { return exp(x); }
-__device__ __forceinline__ float bp_log(float x) { return logf(x); }
-__device__ __forceinline__ double bp_log(double x) { return log(x); }
-
 template <class T>
 struct BP_F {
   using V = typename Vec2<T>::type;
@@ -914,7 +907,7 @@ struct BP_F {
   const V *lc;
   V *ln;
   const V *prior;
-  T p00, p01, p10, p11;
+  BpPsi<T> psi;
   using Acc = int32_t;
   static constexpr int kLaneEdges = 5;  // 2 % faster per pass than 6 at scale 24
   __device__ __forceinline__ bool cond(int) const { return true; }
@@ -929,13 +922,9 @@ struct BP_F {
     else
       out = ln[d];
     if (k > 0) {
-      const V l = lc[d], pr = prior[d];
-      const T lm = l.x > l.y ? l.x : l.y;
-      const T a0 = pr.x * bp_exp(l.x - lm), a1 = pr.y * bp_exp(l.y - lm);
-      const T b0 = p00 * a0 + p01 * a1, b1 = p10 * a0 + p11 * a1;
-      const T lz = bp_log(b0 + b1);
-      out.x += (T)k * (bp_log(b0) - lz);
-      out.y += (T)k * (bp_log(b1) - lz);
+      const V add = bp_message(psi, prior[d], lc[d], k);
+      out.x += add.x;
+      out.y += add.y;
     }
     if (in_f || k > 0) ln[d] = out;
     return k > 0;
@@ -943,9 +932,23 @@ struct BP_F {
 };
 
 template <class T>
+void run_bp_counts(pm_graph *g, const T *d_prior, const T *psi, int iters, T *d_out);
+
+// Whole graphs: the counts by peeling (pm_bp.cu).  A partition's ranks hold
+// only their own in-edges and exchange the frontier, so they pull each pass;
+// so does a call that finds no memory for the counts (12 n bytes more).
+template <class T>
 void run_bp(pm_graph *g, const T *d_prior, const T *psi, int iters, T *d_out) {
   using V = typename Vec2<T>::type;
   Engine &E = g->E;
+  if (!g->is_part) {
+    try {
+      run_bp_counts<T>(g, d_prior, psi, iters, d_out);
+      return;
+    } catch (const Failure &f) {
+      if (f.status != PM_ERR_OOM) throw;
+    }
+  }
   const int64_t n = g->n;
   V *lc = (V *)g->scratch_buf(0, (size_t)n * sizeof(V));
   V *ln = (V *)g->scratch_buf(1, (size_t)n * sizeof(V));
@@ -962,7 +965,7 @@ void run_bp(pm_graph *g, const T *d_prior, const T *psi, int iters, T *d_out) {
                  PM_CUDA(cudaMemsetAsync(E.d_cnt, 0, sizeof(Counters), E.stream));
                  E.prof.begin("bp", E.stream);
                  launch_pull_reduce<int>(
-                     E, BP_F<T>{fa, a, b, (const V *)d_prior, psi[0], psi[1], psi[2], psi[3]}, nullptr,
+                     E, BP_F<T>{fa, a, b, (const V *)d_prior, BpPsi<T>{psi[0], psi[1], psi[2], psi[3]}}, nullptr,
                      fb, E.d_cnt);
                  E.prof.end(E.stream);
                  part_exchange_bits(g, fb);  // a partition: the next frontier of every rank
