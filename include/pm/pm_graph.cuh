@@ -99,6 +99,15 @@ struct AdjBuf {
   }
 };
 
+// The degree-sorted copy of one adjacency (pm_sorted.cuh): rows longest
+// first, sources as positions in that order; built on first use.
+struct SortedView;
+struct SortedAdj {
+  DevBuf order, odeg, off, ids, w, deg, pieces, pfirst, partials, done;
+  int64_t slots = 0;
+  std::shared_ptr<SortedView> view;
+};
+
 }  // namespace pm
 
 struct pm_graph : pm::IdleFreeBase {
@@ -113,6 +122,7 @@ struct pm_graph : pm::IdleFreeBase {
   pm::DevBuf w_i32_out, w_i32_in, w_f32_out, w_f32_in;
   pm::DevBuf w_f32_pair_in;   // {CSC source, float weight} per CSC slot, built on first use
   pm::DevBuf w_f32_pair_out;  // {CSR destination, float weight} per CSR slot, likewise
+  pm::SortedAdj sorted_in, sorted_out;
   pm::Engine E;
   cudaStream_t own_stream = nullptr;  // created with the handle; E.stream may be a caller's
   pm::DevBuf cnt, bits0, bits1, queue0, queue1, defer, hubs, partials, hdone;

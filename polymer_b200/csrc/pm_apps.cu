@@ -805,7 +805,14 @@ __global__ void k_pr_init(T *pc, T *pn, T *c, const int32_t *out_off, int64_t n)
 __global__ void k_copy_daux(const Counters *cnt, double *dst) { *dst = cnt->daux; }
 
 template <class T>
+bool run_pagerank_sorted(pm_graph *g, int iters, double damping, T *d_out, double *d_resid);
+
+// Whole graphs sum over the degree-sorted copy (pm_sorted.cu); a partition,
+// whose ranks exchange ranges of vertices, and a handle without room for the
+// copy pull over the CSC.
+template <class T>
 void run_pagerank(pm_graph *g, int iters, double damping, T *d_out, double *d_resid) {
+  if (run_pagerank_sorted<T>(g, iters, damping, d_out, d_resid)) return;
   Engine &E = g->E;
   const int64_t n = g->n;
   T *pc = (T *)g->scratch_buf(0, (size_t)n * sizeof(T));
@@ -870,7 +877,11 @@ struct SPMV_F {
 // T = float: the FP32 storage and sums of the benchmark; T = double: the same
 // iteration in FP64, the yardstick for the FP32 result's error.
 template <class T>
+bool run_spmv_sorted(pm_graph *g, const T *d_x0, int iters, T *d_y, double *d_norm);
+
+template <class T>
 void run_spmv(pm_graph *g, const T *d_x0, int iters, T *d_y, double *d_norm) {
+  if (run_spmv_sorted<T>(g, d_x0, iters, d_y, d_norm)) return;
   Engine &E = g->E;
   const int64_t n = g->n;
   T *x = (T *)g->scratch_buf(0, (size_t)n * sizeof(T));

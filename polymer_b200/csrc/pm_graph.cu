@@ -355,6 +355,8 @@ void permute_weights_f32(pm_graph *g) {
   const int64_t m = g->m;
   g->w_f32_pair_in.reset();  // rebuilt from the new weights on first use
   g->w_f32_pair_out.reset();
+  g->sorted_in.w.reset();
+  g->sorted_out.w.reset();
   g->w_f32_in.alloc((size_t)std::max<int64_t>(m, 1) * 4);
   if (m)
     PM_LAUNCH(k_gather<float>, grid1d(m), 256, 0, g->E.stream, g->w_f32_out.as<float>(),
