@@ -70,8 +70,10 @@ struct SortedView {
   int64_t blocks() const { return np + (warps() + kSortThreads / 32 - 1) / (kSortThreads / 32); }
 };
 
-// The sum of f.edge over slots e, e + STRIDE, ... below e1: U id loads, then
-// U gathers in flight; the remainder is one predicated step.
+// The sum of f.edge over slots e, e + STRIDE, ... below e1: four id loads, then
+// four gathers in flight, their values added in pairs (a quarter of the
+// dependent additions, and of their rounding); the remainder is one predicated
+// step.
 template <bool W, int STRIDE, class F>
 __device__ __forceinline__ typename F::Acc sorted_sum(const SortedView &a, const F &f, int e, int e1) {
   using Acc = typename F::Acc;
@@ -85,8 +87,10 @@ __device__ __forceinline__ typename F::Acc sorted_sum(const SortedView &a, const
       s[u] = __ldcs(a.ids + e + u * STRIDE);
       if constexpr (W) w[u] = __ldcs(a.w + e + u * STRIDE);
     }
+    Acc v[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) acc = f.combine(acc, f.edge(s[u], W ? w[u] : 0.0f));
+    for (int u = 0; u < U; ++u) v[u] = f.edge(s[u], W ? w[u] : 0.0f);
+    acc = f.combine(acc, f.combine(f.combine(v[0], v[1]), f.combine(v[2], v[3])));
   }
   if (e < e1) {
 #pragma unroll
