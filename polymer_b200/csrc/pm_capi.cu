@@ -571,11 +571,12 @@ pm_status pm_bfs(pm_graph *g, int32_t src, int32_t *parents, int32_t *depth, uin
     check_mem(mem);
     need(src >= 0 && src < g->n, "source out of range");
     const size_t bytes = (size_t)g->n * 4;
-    int32_t *dp = (int32_t *)g->scratch_buf(kSlotOut0, bytes);
-    int32_t *dd = (int32_t *)g->scratch_buf(kSlotOut1, bytes);
+    const bool dev = mem == PM_MEM_DEVICE;
+    int32_t *dp = dev && parents ? parents : (int32_t *)g->scratch_buf(kSlotOut0, bytes);
+    int32_t *dd = dev && depth ? depth : (int32_t *)g->scratch_buf(kSlotOut1, bytes);
     run_bfs(g, src, dp, dd, threshold < 0 ? g->m / g->E.tune.bfs_div : threshold, stats);
-    if (parents) from_device(g, parents, dp, bytes, mem);
-    if (depth) from_device(g, depth, dd, bytes, mem);
+    if (!dev && parents) from_device(g, parents, dp, bytes, mem);
+    if (!dev && depth) from_device(g, depth, dd, bytes, mem);
     finish(g);
   });
 }
