@@ -1398,6 +1398,10 @@ struct Profiler {
     std::vector<Rec> &v = capturing ? captured : recs;
     if (!v.empty()) record(v.back().b, s);
   }
+  // The last bracket covered this many passes (known only after the call).
+  void set_passes(int passes) {
+    if (enabled && !recs.empty()) recs.back().passes = passes;
+  }
   void add(const Rec &r) {
     float ms = 0.f;
     PM_CUDA(cudaEventElapsedTime(&ms, r.a, r.b));

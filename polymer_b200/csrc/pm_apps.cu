@@ -131,15 +131,20 @@ __global__ void k_iota32(int32_t *a, int64_t n) {
 }
 
 void run_cc_union_find(pm_graph *g, int32_t *d_labels, pm_traversal_stats *st);
+void run_cc_rounds(pm_graph *g, int32_t *d_labels, int64_t threshold, pm_traversal_stats *st);
 
 // Symmetric whole-graph handles take the union-find of pm_cc.cu (the same
-// labels, PM_TUNE_CC_MODE 0, the default); directed graphs, partitions and
-// mode 1 run the reference's label propagation below.
+// labels, PM_TUNE_CC_MODE 0, the default); directed graphs and mode 1 run the
+// reference's label propagation with every round in one launch (pm_min.cu);
+// partitions, warp-aggregated pushes and staged pulls run its host loop below.
 void run_cc(pm_graph *g, int32_t *d_labels, int64_t threshold, pm_traversal_stats *st) {
   if (g->symmetric && !g->is_part && g->E.tune.cc_mode == 0) {
     run_cc_union_find(g, d_labels, st);
     return;
   }
+  if (!g->is_part && !g->E.tune.push_agg && !g->E.tune.pull_stage &&
+      unless_no_memory([&] { run_cc_rounds(g, d_labels, threshold, st); }))
+    return;
   Engine &E = g->E;
   VertexSubset cur = g->subset(0), next = g->subset(1);
   PM_LAUNCH(k_iota32, E.grid_for(g->n, 256, 16), 256, 0, E.stream, d_labels, g->n);
@@ -528,9 +533,16 @@ static void run_bellman_ford_delta(pm_graph *g, int32_t *d_dist, int64_t thresho
   }
 }
 
+void run_bellman_ford_rounds(pm_graph *g, int32_t src, int32_t *d_dist, int64_t threshold, pm_traversal_stats *st);
+
+// The default rounds of a whole graph run in one launch (pm_min.cu); the
+// other schedules and partitions run the host loops here.
 void run_bellman_ford(pm_graph *g, int32_t src, int32_t *d_dist, int64_t threshold,
                       pm_traversal_stats *st) {
   Engine &E = g->E;
+  if (!g->is_part && E.tune.bf_dense == 2 && E.tune.bf_delta == 0 && !E.tune.push_agg &&
+      unless_no_memory([&] { run_bellman_ford_rounds(g, src, d_dist, threshold, st); }))
+    return;
   VertexSubset cur = g->subset(0), next = g->subset(1);
   PM_LAUNCH(k_bf_init, E.grid_for(g->n, 256, 16), 256, 0, E.stream, d_dist, g->n, src);
   subset_single(E, cur, src);

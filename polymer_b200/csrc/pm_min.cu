@@ -1,0 +1,180 @@
+// pm_min.cu -- minimum propagation on whole graphs, every round in one
+// cooperative launch: BellmanFord (BF_F numa-BellmanFord.C:61-95, loop
+// 166-211) and the label propagation of Components on directed graphs (CC_F
+// numa-Components.C:55-119, loop 233-281).  The options of these applications
+// (pull or DENSE_FORWARD rounds, delta-stepping, warp-aggregated pushes) and
+// partitions run the host loops of pm_apps.cu.
+//
+// A round pushes val[s] (+ weight) over the frontier's out-edges from queues
+// whose rows are cut to bounded pieces (pm_rounds.cuh); the next frontier is
+// what fell.  Rounds below the threshold learn that from the atomics' results
+// (a stamp keeps a vertex from being queued twice).  Rounds at or above it
+// issue atomics without results, skipped when the target's value as this SM
+// last saw it is already no larger (values only fall, so one seen earlier is
+// never below the current one), and find what fell by comparing with a copy
+// taken at the round's start.
+//
+// What bounds it: the gathers of the targets' values in the one or two rounds
+// that push most of the graph (200 G edges/s), and, on small graphs, the
+// barriers.  BellmanFord on the symmetrised 2^22-vertex, 128 M-edge R-MAT
+// (weights 1..22): 1.69 ms as a host loop -> 1.16 ms here.
+#include "pm_rounds.cuh"
+
+namespace pm {
+
+struct MinWork {
+  int32_t *val, *before, *stamp;
+  RoundQueue q[2];
+  RoundCount *count;  // three slots, level % 3
+  pm_traversal_stats *stats;
+};
+
+// W: val + weight from the source src (BellmanFord); otherwise every vertex
+// starts with its id and in the frontier (labels).
+template <bool W>
+__global__ void __launch_bounds__(kRoundThreads, 2) k_min_rounds(GraphView g, const int32_t *__restrict__ weight,
+                                                                 MinWork w, int32_t src, int64_t threshold) {
+  cg::grid_group grid = cg::this_grid();
+  const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, gsize = (int64_t)gridDim.x * blockDim.x;
+  constexpr int64_t kTile = (int64_t)kRoundThreads * kStep;
+  for (int64_t v = gtid; v < g.n; v += gsize) {
+    w.val[v] = W ? (v == src ? 0 : kDevBFInf) : (int32_t)v;
+    w.stamp[v] = 0;
+  }
+  if (W && blockIdx.x == 0 && threadIdx.x < 32) round_start(g, src, w.q[0], w.count);
+  // the vertices of the block's tiles for which in(v) holds become the frontier
+  // q, counted in c
+  auto collect = [&](auto &&in, const RoundQueue &q, RoundCount *c) {
+    unsigned long long size = 0, edges = 0;
+    for (int64_t base = blockIdx.x * kTile; base < g.n; base += gridDim.x * kTile) {
+      bool act[kStep];
+      int v[kStep], deg[kStep];
+#pragma unroll
+      for (int i = 0; i < kStep; ++i) {
+        const int64_t x = base + i * kRoundThreads + threadIdx.x;
+        v[i] = (int)min(x, (int64_t)g.n - 1);
+        act[i] = in(v[i]) && x < g.n;
+      }
+#pragma unroll
+      for (int i = 0; i < kStep; ++i) {
+        deg[i] = act[i] ? __ldg(g.out.off + v[i] + 1) - __ldg(g.out.off + v[i]) : 0;
+        size += act[i];
+        edges += (unsigned)deg[i];
+      }
+      round_append_block(act, v, deg, q, c);
+    }
+    round_count_add(size, edges, c);
+  };
+  if (!W) collect([](int) { return true; }, w.q[0], w.count);
+  grid.sync();
+  // a source's value as its piece or row is taken: one lowered later in the
+  // round is in the next frontier and pushes again
+  auto value_of = [&](int s) { return *((volatile int32_t *)w.val + s); };
+  pm_traversal_stats st{};
+  for (int32_t level = 1;; ++level) {
+    RoundCount *cur = w.count + (level - 1) % 3, *nxt = w.count + level % 3;
+    const RoundCount f = round_read(cur);
+    const unsigned long long fsize = f.size, fedges = f.edges;
+    if (fsize == 0 || st.rounds > (int64_t)g.n + 1) break;
+    const bool dense = (long long)(fsize + fedges) >= threshold;
+    const RoundQueue &q = w.q[(level - 1) & 1], &qn = w.q[level & 1];
+    st.rounds++;
+    st.dense_rounds += dense;
+    st.edges_visited += (int64_t)fedges;
+    if (gtid == 0) w.count[(level + 1) % 3] = RoundCount{};
+    if (dense) {
+      for (int64_t v0 = gtid; v0 < g.n; v0 += kStep * gsize) {  // four loads in flight
+        int32_t x[kStep];
+#pragma unroll
+        for (int i = 0; i < kStep; ++i) x[i] = w.val[min(v0 + i * gsize, (int64_t)g.n - 1)];
+#pragma unroll
+        for (int i = 0; i < kStep; ++i)
+          if (v0 + i * gsize < g.n) w.before[v0 + i * gsize] = x[i];
+      }
+      grid.sync();
+      round_push(g, q, f.rows, f.pieces, value_of,
+                 [&](const int (&x)[kStep], const int (&e)[kStep], const int (&d)[kStep], const bool (&ok)[kStep]) {
+                   int32_t nv[kStep], seen[kStep];
+#pragma unroll
+                   for (int u = 0; u < kStep; ++u) nv[u] = x[u] + (W && ok[u] ? __ldg(weight + e[u]) : 0);
+#pragma unroll
+                   for (int u = 0; u < kStep; ++u) seen[u] = ok[u] ? __ldca(w.val + d[u]) : 0;
+#pragma unroll
+                   for (int u = 0; u < kStep; ++u)
+                     if (ok[u] && nv[u] < seen[u]) atomicMin(w.val + d[u], nv[u]);
+                 });
+      grid.sync();
+      collect([&](int v) { return __ldcs(w.val + v) < __ldcs(w.before + v); }, qn, nxt);
+    } else {
+      unsigned long long size = 0, edges = 0;
+      round_push(g, q, f.rows, f.pieces, value_of,
+                 [&](const int (&x)[kStep], const int (&e)[kStep], const int (&d)[kStep], const bool (&ok)[kStep]) {
+                   bool act[kStep];
+                   int deg[kStep];
+                   int32_t nv[kStep];
+#pragma unroll
+                   for (int u = 0; u < kStep; ++u) {
+                     nv[u] = x[u] + (W && ok[u] ? __ldg(weight + e[u]) : 0);
+                     act[u] = ok[u] && nv[u] < *((volatile int32_t *)w.val + d[u]);
+                   }
+#pragma unroll
+                   for (int u = 0; u < kStep; ++u) act[u] = act[u] && nv[u] < atomicMin(w.val + d[u], nv[u]);
+#pragma unroll
+                   for (int u = 0; u < kStep; ++u) act[u] = act[u] && atomicExch(w.stamp + d[u], level) != level;
+#pragma unroll
+                   for (int u = 0; u < kStep; ++u) {
+                     deg[u] = act[u] ? __ldg(g.out.off + d[u] + 1) - __ldg(g.out.off + d[u]) : 0;
+                     size += act[u];
+                     edges += (unsigned)deg[u];
+                   }
+                   round_append(act, d, deg, qn, nxt);
+                 });
+      round_count_add(size, edges, nxt);
+    }
+    grid.sync();
+  }
+  if (gtid == 0) *w.stats = st;
+}
+
+template <bool W>
+static pm_traversal_stats run_min(pm_graph *g, const int32_t *weight, int32_t src, int32_t *d_val, int64_t threshold,
+                                  const char *tag) {
+  Engine &E = g->E;
+  const size_t pieces = round_pieces(g->m);
+  MinWork w;
+  w.val = d_val;
+  w.before = (int32_t *)g->scratch_buf(37, (size_t)g->n * 4);
+  w.stamp = E.defer;
+  int2 *pc = (int2 *)g->scratch_buf(0, 2 * pieces * sizeof(int2));
+  for (int k = 0; k < 2; ++k) {
+    w.q[k].rows = g->subset(k).queue;
+    w.q[k].pieces = pc + k * pieces;
+  }
+  w.count = (RoundCount *)g->scratch_buf(30, 3 * sizeof(RoundCount));
+  static_assert(sizeof(pm_traversal_stats) <= 3 * sizeof(Counters), "written to the pinned counter words");
+  w.stats = (pm_traversal_stats *)E.h_cnt;  // pinned: the kernel writes it over the bus
+  if (!W) PM_CUDA(cudaMemsetAsync(w.count, 0, 3 * sizeof(RoundCount), E.stream));
+  static const int per_sm = round_occupancy(k_min_rounds<W>);
+  E.prof.begin(tag, E.stream);
+  PM_LAUNCH_COOP((k_min_rounds<W>), round_grid(E, per_sm), kRoundThreads, E.stream, E.g, weight, w, src, threshold);
+  E.prof.end(E.stream);
+  PM_CUDA(cudaStreamSynchronize(E.stream));
+  const pm_traversal_stats st = *w.stats;
+  E.prof.set_passes((int)st.rounds);
+  return st;
+}
+
+void run_bellman_ford_rounds(pm_graph *g, int32_t src, int32_t *d_dist, int64_t threshold, pm_traversal_stats *st) {
+  pm_traversal_stats s = run_min<true>(g, g->w_i32_out.as<int32_t>(), src, d_dist, threshold, "bellman_ford");
+  if (s.rounds > g->n + 1) fail(PM_ERR_INVALID_ARG, "BellmanFord did not converge");
+  s.reached = 1;
+  if (st) *st = s;
+}
+
+void run_cc_rounds(pm_graph *g, int32_t *d_labels, int64_t threshold, pm_traversal_stats *st) {
+  pm_traversal_stats s = run_min<false>(g, nullptr, -1, d_labels, threshold, "cc");
+  s.reached = g->n;
+  if (st) *st = s;
+}
+
+}  // namespace pm

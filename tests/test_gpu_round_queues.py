@@ -52,6 +52,16 @@ def test_traversals_exact(pm, oracle, n, symmetric):
                 assert np.array_equal(pm.BellmanFord(g, s, threshold=thr), oracle.dijkstra(og, w, s)), (thr, s)
 
 
+def test_profiled_rounds_are_counted(pm, oracle):
+    og = oracle.rmat_graph(11, 8, symmetric=True)
+    s = int(oracle.pick_sources(og, 1)[0])
+    with pm.Graph.from_csr(og.off, og.idx, symmetric=True, weights=oracle.weights_int(og)) as g:
+        g.profile(True)
+        _, st = pm.BellmanFord(g, s, stats=True)
+        ms, passes = g.profile_read("bellman_ford", reset=True)
+        assert passes == st["rounds"] and ms > 0
+
+
 def test_device_outputs_and_odd_alignment(pm, oracle):
     """Results written straight into CUDA buffers, also 4-byte aligned ones."""
     import torch
