@@ -8,35 +8,39 @@
 // that yields that minimum gives the reference's labels bit for bit.
 //
 // This file computes it with a concurrent union-find in the scheme of
-// Afforest (Sutton, Ben-Nun and Barak, IPDPS 2018):
-//   1. every vertex links to its first kSampleRounds neighbours (one round
-//      per neighbour index, a compression after each);
-//   2. the root shared by most of kModeSamples fixed vertices is taken as
-//      the largest intermediate component L;
-//   3. every vertex whose root is not L links to its remaining neighbours.
-//      A vertex of L skips them: an edge between L and another component
-//      is also stored the other way round (the graph is symmetric), and the
-//      other endpoint, not in L, links it; an edge inside L needs nothing;
-//   4. a last compression points every vertex at its root.
-// Links always hang the larger root under the smaller one with a CAS, so
-// parent[v] <= v holds throughout, a root is the least id of its tree, and
-// the final root of each component is its minimum vertex id: exactly the
-// labels of the propagation.  The parent array is the caller's label array.
+// Afforest (Sutton, Ben-Nun and Barak, IPDPS 2018), in one cooperative launch:
+//   1. every vertex hangs under its first neighbour when that is smaller (its
+//      own entry only: no atomics; rows are usually sorted, so this is mostly
+//      the least neighbour), and the trees are compressed;
+//   2. every vertex links to its second neighbour, and the trees are
+//      compressed again;
+//   3. the root shared by most of kModeSamples spread vertices is taken as the
+//      largest intermediate component L;
+//   4. every vertex not under L links to all its neighbours.  A vertex of L
+//      skips them: an edge between L and another component is also stored the
+//      other way round (the graph is symmetric), and the other endpoint, not
+//      in L, links it; an edge inside L needs nothing;
+//   5. a last compression points every vertex at its root.
+// Links always hang the larger root under the smaller one (with a CAS in steps
+// 2 and 4), so parent[v] <= v holds throughout, a root is the least id of its
+// tree, and the final root of each component is its minimum vertex id: exactly
+// the labels of the propagation.  The parent array is the caller's label array.
 // Label propagation stays available (tunable PM_TUNE_CC_MODE = 1) and is
 // what directed and partitioned handles use.
+//
+// What bounds it: the dependent reads id -> parent -> parent of a few million
+// vertices.  Each thread therefore follows kStep vertices side by side, and
+// the compressions read parents through L1 (a stale parent is an ancestor
+// too), where most trees end.  Symmetrised 2^22-vertex, 128 M-edge R-MAT:
+// 380 us as eight kernels (init 5, sampling 97 + 42, compressions 101 + 40 +
+// 39, mode 18, rest 35) -> 213 us.
 #include <algorithm>
 
-#include "pm_graph.cuh"
+#include "pm_rounds.cuh"
 
 namespace pm {
 
-constexpr int kSampleRounds = 2;
-constexpr int kModeSamples = 1024;
-constexpr int kSlotCcMode = 31;  // scratch slot of the largest component's root
-
-#define GRID_STRIDE(i, count)                                                       \
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (count);     \
-       i += (int64_t)gridDim.x * blockDim.x)
+constexpr int kModeSamples = kRoundThreads;
 
 __device__ __forceinline__ int32_t ld_parent(const int32_t *p, int32_t v) {
   return *((volatile const int32_t *)p + v);
@@ -56,120 +60,167 @@ __device__ __forceinline__ void uf_link(int32_t *parent, int32_t u, int32_t v) {
   }
 }
 
-__device__ __forceinline__ int32_t uf_root(const int32_t *parent, int32_t v) {
-  int32_t p = ld_parent(parent, v);
-  while (true) {
-    const int32_t q = ld_parent(parent, p);
-    if (q == p) return p;
-    p = q;
-  }
-}
+// Steps a compression takes through L1 without storing: most trees are no
+// deeper.  Past them every thread stores its jumps and reads past L1, so that
+// all chains shorten together (pointer doubling): a path of n vertices in id
+// order takes log n steps, not n.
+constexpr int kShallow = 8;
 
-__global__ void k_uf_init(int32_t *parent, int64_t n) {
-  GRID_STRIDE(v, n) parent[v] = (int32_t)v;
-}
-
-// Round r of the sampling: v links to its r-th neighbour (when it has one).
-__global__ void k_uf_sample(GraphView g, int32_t *parent, int r, unsigned long long *edges) {
-  unsigned long long mine = 0;
-  GRID_STRIDE(v, g.n) {
-    const int32_t o0 = __ldg(g.out.off + v), o1 = __ldg(g.out.off + v + 1);
-    if (o1 - o0 > r) {
-      uf_link(parent, (int32_t)v, checked_id(g, __ldg(g.out.idx + o0 + r)));
-      ++mine;
+// parent[v] := root of v, for every v.  Writes only v's own entry; a reader of
+// parent[v] meanwhile sees either the old value or the root, both ancestors.
+__device__ __forceinline__ void uf_compress(int32_t *parent, int64_t n) {
+  const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, gsize = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t v0 = gtid; v0 < n; v0 += kStep * gsize) {
+    int32_t old[kStep], p[kStep], q[kStep];
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) old[u] = p[u] = __ldca(parent + min(v0 + u * gsize, n - 1));
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) q[u] = __ldca(parent + p[u]);
+    for (int step = 0;; ++step) {
+      bool more = false;
+#pragma unroll
+      for (int u = 0; u < kStep; ++u)
+        if (p[u] != q[u]) {
+          p[u] = q[u];
+          if (step < kShallow) {
+            q[u] = __ldca(parent + q[u]);
+          } else {  // a long chain: publish the jump, read what others published
+            if (v0 + u * gsize < n) parent[v0 + u * gsize] = p[u];
+            q[u] = ld_parent(parent, q[u]);
+          }
+          more |= p[u] != q[u];
+        }
+      if (!more) break;
     }
-  }
-  mine = warp_sum(mine);
-  if (lane_id() == 0 && mine) atomicAdd(edges, mine);
-}
-
-// parent[v] := root of v.  Writes only v's own entry; a concurrent reader of
-// parent[v] sees either the old value or the root, both ancestors of v.
-__global__ void k_uf_compress(int32_t *parent, int64_t n) {
-  GRID_STRIDE(v, n) {
-    const int32_t r = uf_root(parent, (int32_t)v);
-    if (ld_parent(parent, (int32_t)v) != r) parent[v] = r;
+#pragma unroll
+    for (int u = 0; u < kStep; ++u)
+      if (v0 + u * gsize < n && p[u] != old[u]) parent[v0 + u * gsize] = p[u];
   }
 }
 
 // The root most of kModeSamples spread vertices share (ties: the smaller
-// root), one CTA of kModeSamples threads; the vertices are v = i * n / S.
-__global__ void __launch_bounds__(kModeSamples) k_uf_mode(const int32_t *parent, int64_t n, int32_t *mode) {
+// root), by every block for itself; the vertices are v = i * n / S.
+__device__ __forceinline__ int32_t uf_mode(const int32_t *parent, int64_t n) {
   __shared__ int32_t s_root[kModeSamples];
   __shared__ unsigned long long s_best;
   const int i = threadIdx.x;
-  const int64_t v = (int64_t)i * n / kModeSamples;
-  s_root[i] = uf_root(parent, (int32_t)v);
+  const int32_t root = __ldca(parent + (int64_t)i * n / kModeSamples);  // compressed: its parent is its root
+  s_root[i] = root;
   if (i == 0) s_best = ~0ull;
   __syncthreads();
   int cnt = 0;
-  for (int j = 0; j < kModeSamples; ++j) cnt += s_root[j] == s_root[i];
+#pragma unroll 8
+  for (int j = 0; j < kModeSamples; ++j) cnt += s_root[j] == root;
   // key: larger count first, then smaller root
-  const unsigned long long key = ((unsigned long long)(kModeSamples - cnt) << 32) | (uint32_t)s_root[i];
-  atomicMin(&s_best, key);
+  const unsigned long long key = ((unsigned long long)(kModeSamples - cnt) << 32) | (uint32_t)root;
+  if (key < s_best) atomicMin(&s_best, key);
   __syncthreads();
-  if (i == 0) *mode = (int32_t)(uint32_t)(s_best & 0xffffffffull);
+  return (int32_t)(uint32_t)(s_best & 0xffffffffull);
 }
 
-// Step 3: a warp takes 32 vertices; each vertex outside the largest
-// component with neighbours past the sampled ones has them linked by the
-// whole warp, one vertex after another.
-__global__ void k_uf_rest(GraphView g, int32_t *parent, const int32_t *mode, unsigned long long *edges) {
+__global__ void __launch_bounds__(kRoundThreads, 2) k_uf(GraphView g, int32_t *parent, unsigned long long *edges) {
+  cg::grid_group grid = cg::this_grid();
   const int lane = lane_id();
-  const int32_t L = *mode;
+  const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, gsize = (int64_t)gridDim.x * blockDim.x;
+  const int64_t n = g.n;
+  if (gtid == 0) *edges = 0;
   unsigned long long mine = 0;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; base < g.n;
-       base += warps * 32) {
-    const int64_t v = base + lane;
-    int32_t o0 = 0, o1 = 0;
-    bool todo = false;
-    if (v < g.n) {
-      o0 = __ldg(g.out.off + v) + kSampleRounds;
-      o1 = __ldg(g.out.off + v + 1);
-      todo = o1 > o0 && uf_root(parent, (int32_t)v) != L;
+  // 1. first neighbours
+  for (int64_t v0 = gtid; v0 < n; v0 += kStep * gsize) {
+    int32_t o0[kStep], o1[kStep], d[kStep];
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      const int64_t v = min(v0 + u * gsize, n - 1);
+      o0[u] = __ldg(g.out.off + v);
+      o1[u] = __ldg(g.out.off + v + 1);
     }
-    unsigned bal = __ballot_sync(0xffffffffu, todo);
-    while (bal) {
-      const int l = __ffs(bal) - 1;
-      bal &= bal - 1;
-      const int32_t u = (int32_t)(base + l);
-      const int32_t e0 = __shfl_sync(0xffffffffu, o0, l), e1 = __shfl_sync(0xffffffffu, o1, l);
-      for (int32_t e = e0 + lane; e < e1; e += 32) {
-        uf_link(parent, u, checked_id(g, __ldg(g.out.idx + e)));
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) d[u] = o0[u] < o1[u] ? checked_id(g, __ldg(g.out.idx + o0[u])) : INT32_MAX;
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      const int64_t v = v0 + u * gsize;
+      if (v < n) {
+        parent[v] = min(d[u], (int32_t)v);
+        mine += d[u] != INT32_MAX;
+      }
+    }
+  }
+  grid.sync();
+  uf_compress(parent, n);
+  grid.sync();
+  // 2. second neighbours
+  for (int64_t v0 = gtid; v0 < n; v0 += kStep * gsize) {
+    int32_t o0[kStep], o1[kStep], d[kStep], pv[kStep], pd[kStep];
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      const int64_t v = min(v0 + u * gsize, n - 1);
+      o0[u] = __ldg(g.out.off + v) + 1;
+      o1[u] = v0 + u * gsize < n ? __ldg(g.out.off + v + 1) : 0;
+      pv[u] = ld_parent(parent, (int32_t)v);
+    }
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) d[u] = o0[u] < o1[u] ? checked_id(g, __ldg(g.out.idx + o0[u])) : -1;
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) pd[u] = d[u] >= 0 ? ld_parent(parent, d[u]) : 0;
+#pragma unroll
+    for (int u = 0; u < kStep; ++u)
+      if (d[u] >= 0) {
         ++mine;
+        if (pd[u] != pv[u]) uf_link(parent, (int32_t)(v0 + u * gsize), d[u]);
+      }
+  }
+  grid.sync();
+  uf_compress(parent, n);
+  grid.sync();
+  // 3. and 4.: a warp takes 32 * kStep vertices; each vertex outside the
+  // largest component has its neighbours linked by the whole warp
+  const int32_t L = uf_mode(parent, n);
+  grid.sync();  // every block has chosen, from the same trees: they agree on L
+  for (int64_t base = gtid - lane; base < n; base += kStep * gsize) {
+    int32_t p[kStep], o0[kStep], o1[kStep];
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      const int64_t v = min(base + u * gsize + lane, n - 1);
+      p[u] = ld_parent(parent, (int32_t)v);
+      o0[u] = __ldg(g.out.off + v);
+      o1[u] = base + u * gsize + lane < n ? __ldg(g.out.off + v + 1) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      unsigned todo = __ballot_sync(0xffffffffu, o0[u] < o1[u] && p[u] != L);
+      while (todo) {
+        const int l = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int32_t v = (int32_t)(base + u * gsize + l);
+        const int32_t e1 = __shfl_sync(0xffffffffu, o1[u], l);
+        const int32_t first = __shfl_sync(0xffffffffu, o0[u], l);
+        for (int32_t e = first + lane; e < e1; e += 32) {
+          uf_link(parent, v, checked_id(g, __ldg(g.out.idx + e)));
+          mine += e >= first + 2;  // the first two were counted above
+        }
       }
     }
   }
   mine = warp_sum(mine);
   if (lane == 0 && mine) atomicAdd(edges, mine);
+  grid.sync();
+  uf_compress(parent, n);
 }
 
 void run_cc_union_find(pm_graph *g, int32_t *d_labels, pm_traversal_stats *st) {
   Engine &E = g->E;
-  const int64_t n = g->n;
-  E.reset_counters();
   unsigned long long *edges = &E.d_cnt->edges;
-  int32_t *mode = (int32_t *)g->scratch_buf(kSlotCcMode, 16);
-  E.tag = "cc";
-  E.prof.begin(E.tag, E.stream);
-  const int grid = E.grid_for(n, 256, 16);
-  PM_LAUNCH(k_uf_init, grid, 256, 0, E.stream, d_labels, n);
-  for (int r = 0; r < kSampleRounds; ++r) {
-    PM_LAUNCH(k_uf_sample, grid, 256, 0, E.stream, E.g, d_labels, r, edges);
-    PM_LAUNCH(k_uf_compress, grid, 256, 0, E.stream, d_labels, n);
-  }
-  PM_LAUNCH(k_uf_mode, 1, kModeSamples, 0, E.stream, d_labels, n, mode);
-  PM_LAUNCH(k_uf_rest, E.grid_for((n + 31) / 32 * 32, 256, 16), 256, 0, E.stream, E.g, d_labels, mode, edges);
-  PM_LAUNCH(k_uf_compress, grid, 256, 0, E.stream, d_labels, n);
+  static const int per_sm = round_occupancy(k_uf);
+  E.prof.begin("cc", E.stream);
+  PM_LAUNCH_COOP(k_uf, round_grid(E, per_sm), kRoundThreads, E.stream, E.g, d_labels, edges);
   E.prof.end(E.stream);
-  const Counters *h = E.read_counters();
   if (st) {
+    const Counters *h = E.read_counters();
     pm_traversal_stats s{};
-    s.rounds = kSampleRounds + 1;  // union-find passes over the vertices
+    s.rounds = 3;  // union-find passes over the vertices
     s.dense_rounds = 0;
     s.edges_visited = (int64_t)h[0].edges;  // edges linked
-    s.reached = n;
+    s.reached = g->n;
     *st = s;
   }
 }

@@ -52,6 +52,22 @@ def test_traversals_exact(pm, oracle, n, symmetric):
                 assert np.array_equal(pm.BellmanFord(g, s, threshold=thr), oracle.dijkstra(og, w, s)), (thr, s)
 
 
+@pytest.mark.parametrize("n", [1, 2, 31, 2049, 60000])
+def test_union_find_long_chains(pm, oracle, n):
+    """Components by union-find where the trees are as deep as they get: a path
+    in id order, in reverse, two interleaved, and rows in descending order."""
+    for step in (1, 2):
+        a = np.arange(n - step) if n > step else np.zeros(0, np.int64)
+        og = oracle.graph_from_edges(n, a, a + step, symmetric=True)
+        rows = [og.idx[og.off[v]:og.off[v + 1]][::-1] for v in range(n)]
+        flipped = np.concatenate(rows) if n else og.idx
+        for idx in (og.idx, flipped.astype(np.int32)):
+            with pm.Graph.from_csr(og.off, idx, symmetric=True) as g:
+                lab, st = pm.Components(g, stats=True)
+                assert np.array_equal(lab, np.arange(n) % step if n > step else np.arange(n))
+                assert st["edges_visited"] <= og.m
+
+
 def test_profiled_rounds_are_counted(pm, oracle):
     og = oracle.rmat_graph(11, 8, symmetric=True)
     s = int(oracle.pick_sources(og, 1)[0])
