@@ -99,11 +99,20 @@ struct AdjBuf {
   }
 };
 
+// The rows of one adjacency by degree, longest first (pm_sorted.cuh): order,
+// the number of rows of at least kSortCta / kSortLong / kSortShort / 1 edges,
+// and the pieces of kOrderPiece edges of the longest kind; built on first use.
+constexpr int kOrderPiece = 16384;
+struct RowOrder {
+  DevBuf order, pieces;  // positions -> vertices; {vertex, first edge of the piece}
+  int32_t cuts[4] = {0, 0, 0, 0};
+  int32_t npieces = 0;
+};
 // The degree-sorted copy of one adjacency (pm_sorted.cuh): rows longest
 // first, sources as positions in that order; built on first use.
 struct SortedView;
 struct SortedAdj {
-  DevBuf order, odeg, off, ids, w, deg, pieces, pfirst, partials, done;
+  DevBuf odeg, off, ids, w, deg, pieces, pfirst, partials, done;
   int64_t slots = 0;
   std::shared_ptr<SortedView> view;
 };
@@ -122,6 +131,7 @@ struct pm_graph : pm::IdleFreeBase {
   pm::DevBuf w_i32_out, w_i32_in, w_f32_out, w_f32_in;
   pm::DevBuf w_f32_pair_in;   // {CSC source, float weight} per CSC slot, built on first use
   pm::DevBuf w_f32_pair_out;  // {CSR destination, float weight} per CSR slot, likewise
+  pm::RowOrder order_in, order_out;
   pm::SortedAdj sorted_in, sorted_out;
   pm::Engine E;
   cudaStream_t own_stream = nullptr;  // created with the handle; E.stream may be a caller's

@@ -35,11 +35,11 @@ __global__ void k_sort_cuts(const int32_t *deg, int64_t n, int32_t *cuts) {
 // pos = the inverse of order; odeg = out-degrees by position; len = slots of
 // row r < rm, then of slice s (32 times its first, longest row); pieces of
 // row r < rc.  len has rm + slices + 1 entries, pieces rc + 1.
-__global__ void k_sort_tables(const int32_t *order, const int32_t *deg, const int32_t *out_off, int64_t n,
+__global__ void k_sort_tables(const int32_t *order, const int32_t *src_off, const int32_t *out_off, int64_t n,
                               int32_t rc, int32_t rm, int32_t rl, int32_t piece, int32_t *pos, int32_t *odeg,
                               int32_t *len, int32_t *pieces, uint8_t *bdeg) {
   GRID_STRIDE(p, n) {
-    const int32_t v = order[p], d = deg[p];
+    const int32_t v = order[p], d = src_off[v + 1] - src_off[v];
     pos[v] = (int32_t)p;
     odeg[p] = out_off[v + 1] - out_off[v];
     if (p < rm) len[p] = d;
@@ -132,40 +132,79 @@ static void exclusive_sum(const int32_t *in, int32_t *out, int64_t count, cudaSt
   PM_CUDA(cub::DeviceScan::ExclusiveSum(tb.p, tmp, in, out, (int)count, st));
 }
 
+// {vertex, first edge} of each kOrderPiece-edge piece of the rows [0, rc).
+__global__ void k_order_pieces(const int32_t *order, const int32_t *src_off, const int32_t *first, int32_t rc,
+                               int2 *pieces) {
+  GRID_STRIDE(r, rc) {
+    const int32_t v = order[r];
+    for (int32_t k = first[r], e = src_off[v]; k < first[r + 1]; ++k, e += kOrderPiece) pieces[k] = make_int2(v, e);
+  }
+}
+__global__ void k_order_counts(const int32_t *deg, int32_t rc, int32_t *count) {
+  GRID_STRIDE(r, rc + 1) count[r] = r < rc ? (deg[r] + kOrderPiece - 1) / kOrderPiece : 0;
+}
+
+const RowOrder &ensure_row_order(pm_graph *g, bool csr) {
+  RowOrder &o = csr ? g->order_out : g->order_in;
+  if (o.order.p) return o;
+  Engine &E = g->E;
+  cudaStream_t st = E.stream;
+  const Adj &src = csr ? E.g.out : E.g.in;
+  const int64_t n = g->n;
+  int bits = 1;
+  while (bits < 31 && (1ll << bits) <= g->m) ++bits;
+  DevBuf order((size_t)n * 4), key((size_t)n * 4), deg((size_t)n * 4), val((size_t)n * 4), cuts(16);
+  PM_LAUNCH(k_sort_keys, E.grid_for(n, 256, 16), 256, 0, st, src.off, n, key.as<int32_t>(), val.as<int32_t>());
+  size_t tmp = 0;
+  PM_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp, key.as<int32_t>(), deg.as<int32_t>(),
+                                                    val.as<int32_t>(), order.as<int32_t>(), (int)n, 0, bits, st));
+  DevBuf tb(std::max<size_t>(tmp, 16));
+  PM_CUDA(cub::DeviceRadixSort::SortPairsDescending(tb.p, tmp, key.as<int32_t>(), deg.as<int32_t>(),
+                                                    val.as<int32_t>(), order.as<int32_t>(), (int)n, 0, bits, st));
+  PM_LAUNCH(k_sort_cuts, 1, 4, 0, st, deg.as<int32_t>(), n, cuts.as<int32_t>());
+  int32_t h[4];
+  PM_CUDA(cudaMemcpyAsync(h, cuts.p, sizeof h, cudaMemcpyDeviceToHost, st));
+  PM_CUDA(cudaStreamSynchronize(st));
+  const int32_t rc = h[0];
+  int32_t np = 0;
+  if (rc > 0) {
+    DevBuf count((size_t)(rc + 1) * 4), first((size_t)(rc + 1) * 4);
+    PM_LAUNCH(k_order_counts, E.grid_for(rc + 1, 256, 16), 256, 0, st, deg.as<int32_t>(), rc, count.as<int32_t>());
+    exclusive_sum(count.as<int32_t>(), first.as<int32_t>(), rc + 1, st);
+    PM_CUDA(cudaMemcpyAsync(&np, first.as<int32_t>() + rc, 4, cudaMemcpyDeviceToHost, st));
+    PM_CUDA(cudaStreamSynchronize(st));
+    o.pieces.alloc((size_t)np * sizeof(int2));
+    PM_LAUNCH(k_order_pieces, E.grid_for(rc, 256, 16), 256, 0, st, order.as<int32_t>(), src.off, first.as<int32_t>(),
+              rc, o.pieces.as<int2>());
+  }
+  std::copy(h, h + 4, o.cuts);
+  o.npieces = np;
+  o.order = std::move(order);
+  return o;
+}
+
 static void build_sorted(pm_graph *g, bool csr, SortedAdj &b) {
   Engine &E = g->E;
   cudaStream_t st = E.stream;
   const Adj &src = csr ? E.g.out : E.g.in;
   const int64_t n = g->n, m = g->m;
+  const RowOrder &o = ensure_row_order(g, csr);
   SortedView v;
   v.n = (int32_t)n;
   v.piece = piece_edges(m);
-  int bits = 1;
-  while (bits < 31 && (1ll << bits) <= m) ++bits;
-  DevBuf order((size_t)n * 4), odeg((size_t)n * 4), key((size_t)n * 4), deg((size_t)n * 4), pos((size_t)n * 4),
-      cuts(16);
+  v.rc = o.cuts[0];
+  v.rh = o.cuts[1];
+  v.rm = o.cuts[2];
+  v.rl = o.cuts[3];
+  v.order = o.order.as<int32_t>();
+  DevBuf odeg((size_t)n * 4), pos((size_t)n * 4);
   const int grid = E.grid_for(n, 256, 16);
-  PM_LAUNCH(k_sort_keys, grid, 256, 0, st, src.off, n, key.as<int32_t>(), pos.as<int32_t>());
-  size_t tmp = 0;
-  PM_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp, key.as<int32_t>(), deg.as<int32_t>(),
-                                                    pos.as<int32_t>(), order.as<int32_t>(), (int)n, 0, bits, st));
-  DevBuf tb(std::max<size_t>(tmp, 16));
-  PM_CUDA(cub::DeviceRadixSort::SortPairsDescending(tb.p, tmp, key.as<int32_t>(), deg.as<int32_t>(),
-                                                    pos.as<int32_t>(), order.as<int32_t>(), (int)n, 0, bits, st));
-  PM_LAUNCH(k_sort_cuts, 1, 4, 0, st, deg.as<int32_t>(), n, cuts.as<int32_t>());
-  int32_t h[4];
-  PM_CUDA(cudaMemcpyAsync(h, cuts.p, sizeof h, cudaMemcpyDeviceToHost, st));
-  PM_CUDA(cudaStreamSynchronize(st));
-  v.rc = h[0];
-  v.rh = h[1];
-  v.rm = h[2];
-  v.rl = h[3];
   const int64_t rows = v.rm + v.slices();  // entries of off before its end
   DevBuf off((size_t)(rows + 1) * 4), len((size_t)(rows + 1) * 4), pieces((size_t)(v.rc + 1) * 4),
       pfirst((size_t)(v.rc + 1) * 4), bdeg((size_t)std::max(v.rl - v.rm, 1));
   PM_CUDA(cudaMemsetAsync(len.as<int32_t>() + rows, 0, 4, st));
   PM_CUDA(cudaMemsetAsync(pieces.as<int32_t>() + v.rc, 0, 4, st));
-  PM_LAUNCH(k_sort_tables, grid, 256, 0, st, order.as<int32_t>(), deg.as<int32_t>(), E.g.out.off, n, v.rc, v.rm,
+  PM_LAUNCH(k_sort_tables, grid, 256, 0, st, v.order, src.off, E.g.out.off, n, v.rc, v.rm,
             v.rl, v.piece, pos.as<int32_t>(), odeg.as<int32_t>(), len.as<int32_t>(), pieces.as<int32_t>(),
             bdeg.as<uint8_t>());
   exclusive_sum(len.as<int32_t>(), off.as<int32_t>(), rows + 1, st);
@@ -179,7 +218,6 @@ static void build_sorted(pm_graph *g, bool csr, SortedAdj &b) {
       partials((size_t)std::max(np, 1) * 8), done((size_t)std::max(v.rc, 1) * 4);
   PM_CUDA(cudaMemsetAsync(done.p, 0, (size_t)std::max(v.rc, 1) * 4, st));
   v.off = off.as<int32_t>();
-  v.order = order.as<int32_t>();
   v.odeg = odeg.as<int32_t>();
   v.deg = bdeg.as<uint8_t>();
   v.pieces = ptab.as<int4>();
@@ -193,7 +231,6 @@ static void build_sorted(pm_graph *g, bool csr, SortedAdj &b) {
   if (blocks > 0)
     PM_LAUNCH((k_sort_fill<true>), (unsigned)blocks, kSortThreads, 0, st, E.g, v, src.off, src.idx, nullptr,
               pos.as<int32_t>(), ids.as<int32_t>(), nullptr);
-  b.order = std::move(order);
   b.odeg = std::move(odeg);
   b.off = std::move(off);
   b.ids = std::move(ids);

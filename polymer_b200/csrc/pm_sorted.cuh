@@ -212,6 +212,9 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(typename F::Acc) == 4 ? 8
 // memory for the copy: the caller then takes the pull over the CSC.
 const SortedView *ensure_sorted(pm_graph *g, bool csr, bool weighted, SortedView &view);
 
+// The rows of g's in-adjacency (or out-adjacency when csr) by degree.
+const RowOrder &ensure_row_order(pm_graph *g, bool csr);
+
 // y[p] = x[order[p]]: a vector in position order.
 template <class T>
 __global__ void k_to_positions(const T *__restrict__ x, const int32_t *__restrict__ order, int64_t n,
