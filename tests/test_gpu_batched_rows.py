@@ -24,6 +24,21 @@ def _picks(og, k):
     return np.concatenate([special, rest]).astype(np.int32)[:k]
 
 
+@pytest.mark.parametrize("k", [1, 7, 8, 9, 16, 17, 31, 32])
+@pytest.mark.parametrize("heavy", [64, 1024])
+def test_ppr_widths(pm, oracle, k, heavy):
+    og = _og(oracle)
+    seeds = _picks(og, k)
+    with pm.Graph.from_csr(og.off, og.idx) as g:
+        g.set_tunable("heavy_deg", heavy)
+        for iters in (1, 2, 3, 6):
+            want = oracle.ppr(og, seeds, iters)
+            got = pm.PersonalizedPageRank(g, seeds, iters)
+            # the suite's FP32 bound, per column
+            assert (np.abs(got - want).sum(0) <= 1e-5 * np.abs(want).sum(0)).all(), iters
+            assert np.array_equal(pm.PersonalizedPageRank(g, seeds, iters), got)
+
+
 @pytest.mark.parametrize("k", [1, 2, 33, 64])
 @pytest.mark.parametrize("transpose", [False, True])
 def test_multi_source_traversals(pm, oracle, k, transpose):
