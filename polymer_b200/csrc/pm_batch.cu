@@ -33,7 +33,12 @@ using u64 = unsigned long long;
 // fell is in the next frontier either way.
 // ===========================================================================
 constexpr int kLanes = 64;
-constexpr int kBfUnroll = 4;      // pull: in-edges whose row gathers are in flight together per warp
+constexpr int kBfUnroll = 4;      // pull: in-edges whose row gathers are in flight together per half-warp
+// Resident CTAs per SM of the pull: 50 sources on a 1.5 M-vertex, 42 M-edge
+// R-MAT take 8.37 ms with four (58 registers), 7.11 with five, 6.64 with six
+// (40 registers) and 6.75 with eight; a warp per row in vertex order, two
+// 128-byte loads a row, took 8.87 to 9.16.
+constexpr int kBfCtas = 6;
 constexpr int kBfPushUnroll = 2;  // push: out-edges whose target rows are read together per warp
 
 // active -> queue of frontier vertices with out-edges (and their degrees);
@@ -159,100 +164,136 @@ __global__ void __launch_bounds__(256) k_bf_multi_push(const int32_t *__restrict
   }
 }
 
-// Relaxes lanes lo / hi of row v over in-edges [e0, e1) whose sources have
-// active lanes (one warp; thread t owns lanes t and t + 32).
-__device__ __forceinline__ void bf_multi_relax(const int32_t *__restrict__ in_idx,
-                                               const int32_t *__restrict__ w_in, const int32_t *dist,
-                                               const u64 *__restrict__ active, int64_t e0, int64_t e1,
-                                               int32_t &lo, int32_t &hi) {
-  const int lane = lane_id();
-  for (int64_t base = e0; base < e1; base += 32) {
-    const int64_t e = base + lane;
+// The least dist[s] + w over this half-warp's in-edges whose sources have
+// active lanes: 16 edges from e on, then from e + step on, ... below e1.  Half
+// a warp holds a source's row (int4: lanes 4 t .. 4 t + 3 of the 64 on its
+// thread t), so one load brings a row to each half and a step has kBfUnroll
+// rows per half in flight.  All lanes of the warp call it; the halves may have
+// different rows and lengths.
+__device__ __forceinline__ int4 bf_multi_relax(const int32_t *__restrict__ in_idx, const int32_t *__restrict__ w_in,
+                                               const int32_t *dist, const u64 *__restrict__ active, int e, int e1,
+                                               int step) {
+  const int t = lane_id() & 15, quad = t * 4, shift = lane_id() & 16;
+  int4 m = make_int4(kDevBFInf, kDevBFInf, kDevBFInf, kDevBFInf);
+  for (; __any_sync(0xffffffffu, e < e1); e += step) {
     int s = 0;
     u64 act = 0;
     int32_t w = 0;
-    if (e < e1) {
-      s = __ldg(in_idx + e);
+    if (e + t < e1) {
+      s = __ldcs(in_idx + e + t);
       act = __ldg(active + s);
-      w = __ldg(w_in + e);
+      w = __ldcs(w_in + e + t);
     }
-    unsigned todo = __ballot_sync(0xffffffffu, act != 0);
-    // Up to kBfUnroll active in-edges per step: their row gathers are all
-    // issued before the first min consumes one.
-    while (todo) {
-      int32_t vlo[kBfUnroll], vhi[kBfUnroll];
+    unsigned todo = (__ballot_sync(0xffffffffu, act != 0) >> shift) & 0xffffu;
+    while (__any_sync(0xffffffffu, todo != 0u)) {
+      int4 v[kBfUnroll];
+      unsigned on[kBfUnroll];
+      int32_t wj[kBfUnroll];
 #pragma unroll
       for (int u = 0; u < kBfUnroll; ++u) {
         const int j = todo ? __ffs(todo) - 1 : 0;
-        const bool take = todo != 0;
-        todo &= todo - 1;
-        const int sj = __shfl_sync(0xffffffffu, s, j);
-        const u64 aj = shfl_idx(act, j) & (take ? ~0ull : 0ull);
-        const int32_t wj = __shfl_sync(0xffffffffu, w, j);
-        vlo[u] = ((aj >> lane) & 1ull) ? dist[(int64_t)sj * kLanes + lane] + wj : kDevBFInf;
-        vhi[u] = ((aj >> (32 + lane)) & 1ull) ? dist[(int64_t)sj * kLanes + 32 + lane] + wj : kDevBFInf;
+        const bool take = todo != 0u;
+        todo &= todo - 1u;
+        const int sj = __shfl_sync(0xffffffffu, s, j, 16);
+        const unsigned lo = __shfl_sync(0xffffffffu, (unsigned)act, j, 16),
+                       hi = __shfl_sync(0xffffffffu, (unsigned)(act >> 32), j, 16);
+        wj[u] = __shfl_sync(0xffffffffu, w, j, 16);
+        on[u] = take ? ((quad < 32 ? lo >> quad : hi >> (quad - 32)) & 15u) : 0u;
+        v[u] = make_int4(0, 0, 0, 0);
+        if (on[u]) v[u] = *reinterpret_cast<const int4 *>(dist + (int64_t)sj * kLanes + quad);
       }
 #pragma unroll
       for (int u = 0; u < kBfUnroll; ++u) {
-        lo = min(lo, vlo[u]);
-        hi = min(hi, vhi[u]);
+        if (on[u] & 1u) m.x = min(m.x, v[u].x + wj[u]);
+        if (on[u] & 2u) m.y = min(m.y, v[u].y + wj[u]);
+        if (on[u] & 4u) m.z = min(m.z, v[u].z + wj[u]);
+        if (on[u] & 8u) m.w = min(m.w, v[u].w + wj[u]);
       }
     }
   }
+  return m;
+}
+// Both halves' minima of one row, on both.
+__device__ __forceinline__ int4 bf_multi_join(int4 m) {
+  m.x = min(m.x, __shfl_xor_sync(0xffffffffu, m.x, 16));
+  m.y = min(m.y, __shfl_xor_sync(0xffffffffu, m.y, 16));
+  m.z = min(m.z, __shfl_xor_sync(0xffffffffu, m.z, 16));
+  m.w = min(m.w, __shfl_xor_sync(0xffffffffu, m.w, 16));
+  return m;
+}
+
+// The 64-bit mask whose bits 4 t .. 4 t + 3 are the nibble of the half's
+// thread t, on every lane of that half.
+__device__ __forceinline__ u64 bf_multi_mask(unsigned nibble) {
+  const int t = lane_id() & 15;
+  unsigned lo = t < 8 ? nibble << (4 * t) : 0u, hi = t < 8 ? 0u : nibble << (4 * (t - 8));
+#pragma unroll
+  for (int d = 8; d > 0; d >>= 1) {
+    lo |= __shfl_xor_sync(0xffffffffu, lo, d);
+    hi |= __shfl_xor_sync(0xffffffffu, hi, d);
+  }
+  return (u64)lo | ((u64)hi << 32);
 }
 
 constexpr int kBfPiece = 512;  // in-edges of one warp's piece of a heavy row
 
-// Dense round.  Persistent warps take tickets: the first ones are 512-edge
-// pieces of the heavy rows (in-degree > g.heavy_deg; they lower the row with
-// atomicMin and OR the fallen lanes into next_active, which starts at zero),
-// the rest are merge-path row groups whose light rows each warp relaxes in
-// full and whose next_active words it writes.
-__global__ void __launch_bounds__(256) k_bf_multi_pull(GraphView g, const int32_t *__restrict__ w_in,
-                                                       int32_t *dist, const u64 *__restrict__ active,
-                                                       u64 *next_active, int64_t heavy_pieces,
-                                                       Counters *cnt) {
-  const int lane = lane_id();
-  for (;;) {
-    long long t = 0;
-    if (lane == 0) t = (long long)atomicAdd(&cnt->aux, 1ull);
-    t = shfl_idx(t, 0);
-    if (t < heavy_pieces) {
-      const int c = (int)(t / (kChunkEdges / kBfPiece));
-      const int piece = (int)(t % (kChunkEdges / kBfPiece));
-      const int r = __ldg(g.in.hrow + c);
-      const int64_t row_end = __ldg(g.in.off + r + 1);
-      const int64_t e0 = (int64_t)__ldg(g.in.off + r) +
-                         (int64_t)(c - __ldg(g.in.hfirst + r)) * kChunkEdges + (int64_t)piece * kBfPiece;
-      if (e0 >= row_end) continue;
-      const int64_t e1 = min(e0 + kBfPiece, row_end);
-      int32_t lo = kDevBFInf, hi = kDevBFInf;
-      bf_multi_relax(g.in.idx, w_in, dist, active, e0, e1, lo, hi);
-      bool fell_lo = false, fell_hi = false;
-      int32_t *p = dist + (int64_t)r * kLanes + lane;
-      if (lo < *(volatile int32_t *)p) fell_lo = lo < atomicMin(p, lo);
-      if (hi < *(volatile int32_t *)(p + 32)) fell_hi = hi < atomicMin(p + 32, hi);
-      const u64 mask = (u64)__ballot_sync(0xffffffffu, fell_lo) | ((u64)__ballot_sync(0xffffffffu, fell_hi) << 32);
-      if (lane == 0 && mask) atomicOr(next_active + r, mask);
-      continue;
+// Dense round, a warp per item: 512-edge pieces of the heavy rows (in-degree >
+// g.heavy_deg; they lower the row with atomicMin and OR the fallen lanes into
+// next_active, which starts at zero), then the light rows in order of
+// in-degree (order: pm_sorted.cu), a warp for each of [0, rh) and half a warp
+// for each of [rh, rl).  A light row is relaxed in full by its lanes, which
+// write its next_active word.
+__global__ void __launch_bounds__(256, kBfCtas) k_bf_multi_pull(GraphView g, const int32_t *__restrict__ w_in,
+                                                                int32_t *dist, const u64 *__restrict__ active,
+                                                                u64 *next_active, int64_t heavy_pieces,
+                                                                const int32_t *__restrict__ order, int rh, int rl) {
+  const int lane = lane_id(), half = lane >> 4, t = lane & 15;
+  int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (item < heavy_pieces) {
+    const int c = (int)(item / (kChunkEdges / kBfPiece));
+    const int piece = (int)(item % (kChunkEdges / kBfPiece));
+    const int r = __ldg(g.in.hrow + c);
+    const int row_end = __ldg(g.in.off + r + 1);
+    const int64_t first = (int64_t)__ldg(g.in.off + r) + (int64_t)(c - __ldg(g.in.hfirst + r)) * kChunkEdges +
+                          (int64_t)piece * kBfPiece;
+    if (first >= row_end) return;
+    const int e0 = (int)first, e1 = min(row_end - e0, kBfPiece) + e0;
+    const int4 m = bf_multi_join(bf_multi_relax(g.in.idx, w_in, dist, active, e0 + 16 * half, e1, 32));
+    unsigned fell = 0;
+    if (half == 0) {
+      int32_t *p = dist + (int64_t)r * kLanes + 4 * t;
+      const volatile int32_t *seen = p;
+      if (m.x < seen[0] && m.x < atomicMin(p, m.x)) fell |= 1u;
+      if (m.y < seen[1] && m.y < atomicMin(p + 1, m.y)) fell |= 2u;
+      if (m.z < seen[2] && m.z < atomicMin(p + 2, m.z)) fell |= 4u;
+      if (m.w < seen[3] && m.w < atomicMin(p + 3, m.w)) fell |= 8u;
     }
-    const long long grp = t - heavy_pieces;
-    if (grp >= g.in.ngroups) break;
-    const int r0 = __ldg(g.in.gstart + grp), r1 = __ldg(g.in.gstart + grp + 1);
-    for (int v = r0; v < r1; ++v) {
-      const int e0 = __ldg(g.in.off + v), e1 = __ldg(g.in.off + v + 1);
-      if (e1 - e0 > g.heavy_deg) continue;
-      const int32_t old_lo = dist[(int64_t)v * kLanes + lane];
-      const int32_t old_hi = dist[(int64_t)v * kLanes + 32 + lane];
-      int32_t lo = old_lo, hi = old_hi;
-      bf_multi_relax(g.in.idx, w_in, dist, active, e0, e1, lo, hi);
-      const unsigned ch_lo = __ballot_sync(0xffffffffu, lo < old_lo);
-      const unsigned ch_hi = __ballot_sync(0xffffffffu, hi < old_hi);
-      if (lo < old_lo) dist[(int64_t)v * kLanes + lane] = lo;
-      if (hi < old_hi) dist[(int64_t)v * kLanes + 32 + lane] = hi;
-      if (lane == 0) next_active[v] = (u64)ch_lo | ((u64)ch_hi << 32);
-    }
+    const u64 mask = bf_multi_mask(fell);
+    if (lane == 0 && mask) atomicOr(next_active + r, mask);
+    return;
   }
+  item -= heavy_pieces;
+  const bool whole = item < rh;  // the same for the whole warp
+  const int64_t r = whole ? item : rh + 2 * (item - rh) + half;
+  int v = 0, e0 = 0, e1 = 0;
+  bool mine = r < rl;
+  if (mine) {
+    v = __ldg(order + r);
+    e0 = __ldg(g.in.off + v);
+    e1 = __ldg(g.in.off + v + 1);
+    mine = e1 - e0 <= g.heavy_deg;
+    if (!mine) e1 = e0;
+  }
+  if (!__any_sync(0xffffffffu, mine)) return;
+  int4 *row = reinterpret_cast<int4 *>(dist + (int64_t)v * kLanes) + t;
+  const int4 old = *row;
+  int4 m = bf_multi_relax(g.in.idx, w_in, dist, active, whole ? e0 + 16 * half : e0, e1, whole ? 32 : 16);
+  if (whole) m = bf_multi_join(m);
+  const unsigned fell = !mine ? 0u : (m.x < old.x) | (m.y < old.y) << 1 | (m.z < old.z) << 2 | (m.w < old.w) << 3;
+  const bool write = !whole || half == 0;
+  if (write && fell) *row = make_int4(min(m.x, old.x), min(m.y, old.y), min(m.z, old.z), min(m.w, old.w));
+  const u64 mask = bf_multi_mask(fell);
+  if (mine && write && t == 0 && mask) next_active[v] = mask;
 }
 
 __global__ void k_bf_multi_init(int32_t *dist, u64 *active, int64_t n) {
@@ -330,18 +371,16 @@ void run_bf_multi(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_dist_
   void *tmp = g->scratch_buf(5, std::max<size_t>(tmp_bytes, 16));
   PM_LAUNCH(k_bf_multi_init, E.grid_for(n * kLanes, 256, 16), 256, 0, E.stream, dist, act, n);
   PM_LAUNCH(k_bf_multi_seed, 1, 64, 0, E.stream, d_sources, k, dist, act);
-  static const int pull_per_sm = [] {
-    int r = 0;
-    PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_bf_multi_pull, 256, 0));
-    return std::max(r, 1);
-  }();
   static const int push_per_sm = [] {
     int r = 0;
     PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_bf_multi_push, 256, 0));
     return std::max(r, 1);
   }();
   const int64_t heavy_pieces = (int64_t)E.g.in.nchunks * (kChunkEdges / kBfPiece);
-  const int pull_grid = E.persistent_grid((heavy_pieces + E.g.in.ngroups + 7) / 8, pull_per_sm);
+  const RowOrder &o = ensure_row_order(g, false);
+  const int rh = o.cuts[1], rl = o.cuts[3];
+  const int64_t items = heavy_pieces + rh + (rl - rh + 1) / 2;
+  const unsigned pull_grid = (unsigned)((items + 7) / 8);
   const int32_t *w_in = g->w_i32_in.as<int32_t>(), *w_out = g->w_i32_out.as<int32_t>();
   pm_traversal_stats s{};
   E.tag = "bellman_ford_multi";
@@ -358,8 +397,9 @@ void run_bf_multi(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_dist_
     E.prof.begin(E.tag, E.stream);
     PM_CUDA(cudaMemsetAsync(nxt, 0, (size_t)n * 8, E.stream));
     if (dense) {
-      PM_LAUNCH(k_bf_multi_pull, pull_grid, 256, 0, E.stream, E.g, w_in, dist, act, nxt, heavy_pieces,
-                E.d_cnt);
+      if (items > 0)
+        PM_LAUNCH(k_bf_multi_pull, pull_grid, 256, 0, E.stream, E.g, w_in, dist, act, nxt, heavy_pieces,
+                  o.order.as<int32_t>(), rh, rl);
     } else {
       if (q > 0) {
         PM_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, qdeg, qoff, (int)q, E.stream));
