@@ -117,6 +117,14 @@ struct SortedAdj {
   std::shared_ptr<SortedView> view;
 };
 
+// The parts of a disjoint union by position (pm_parts.cu): built on the first
+// call after the parts were set.
+struct PartsLayout {
+  DevBuf pbase, order, deg, odeg, soff, ids;
+  int64_t npos = 0;
+  int state = 0;  // 1 built, -1 not usable for these parts, 0 not built
+};
+
 }  // namespace pm
 
 struct pm_graph : pm::IdleFreeBase {
@@ -144,6 +152,7 @@ struct pm_graph : pm::IdleFreeBase {
   // largest-first order in which persistent kernels take them
   std::vector<int64_t> parts;       // count+1 vertex offsets (host copy); empty if none
   pm::DevBuf parts_vbase, parts_order;
+  pm::PartsLayout parts_layout;
   // 1D vertex partition across processes (pm_graph_create_partition): this
   // handle holds the edges whose destination lies in [part_lo, part_hi)
   // (rank r owns [part_bounds[r], part_bounds[r+1]); part_wbounds are the

@@ -1,14 +1,9 @@
 // pm_batch.cu -- batched workloads: multi-source BellmanFord (64 int32
-// distance lanes per vertex), personalised PageRank for 32 seeds, and PageRank
-// on every part of a disjoint union in one persistent launch (multi-source
-// BFS: pm_msbfs.cu).
-#include <cooperative_groups.h>
-
+// distance lanes per vertex) and personalised PageRank for up to 32 seeds
+// (multi-source BFS: pm_msbfs.cu; the parts of a disjoint union: pm_parts.cu).
 #include <cub/cub.cuh>
 
 #include "pm_sorted.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace pm {
 
@@ -654,102 +649,6 @@ void run_ppr(pm_graph *g, const int32_t *d_seeds, int k, int iters, double dampi
     run_ppr_cols<16>(g, d_seeds, k, iters, damping, d_out);
   else
     run_ppr_cols<kPprCols>(g, d_seeds, k, iters, damping, d_out);
-}
-
-// ===========================================================================
-// Many independent graphs (the parts of a disjoint union) each running
-// PageRank with Polymer's semantics (PR_F / PR_Vertex_F / PR_Vertex_Reset,
-// numa-PageRank.C:64-148, n = the part's own vertex count), all in ONE
-// persistent launch.  Thread-block clusters of kPartCluster CTAs take parts
-// from a work queue, largest first; the CTAs of a cluster split the part's
-// vertices and separate the phases of an iteration with the cluster barrier
-// (barrier.cluster, a hardware barrier: no flag is polled).  One thread per
-// vertex sums its in-edges; the frontier rides in the contribution sign as in
-// run_pagerank.
-// ===========================================================================
-constexpr int kPartCluster = 8;
-constexpr int kPartThreads = 512;
-
-__global__ void __cluster_dims__(kPartCluster, 1, 1) __launch_bounds__(kPartThreads)
-    k_pagerank_parts(GraphView g, const int64_t *__restrict__ vbase, const int32_t *__restrict__ order,
-                     int count, int iters, float damping, float *pc, float *pn, float *c0, float *c1,
-                     float *out, Counters *queue) {
-  cg::cluster_group cluster = cg::this_cluster();
-  __shared__ int s_part;
-  const int rank = (int)cluster.block_rank();
-  const int64_t stride = (int64_t)kPartCluster * kPartThreads;
-  for (;;) {
-    if (rank == 0 && threadIdx.x == 0) s_part = (int)atomicAdd(&queue->aux, 1ull);
-    cluster.sync();
-    const int part = *cluster.map_shared_rank(&s_part, 0);
-    cluster.sync();  // every CTA has read the ticket before the next one is drawn
-    if (part >= count) break;
-    const int p = __ldg(order + part);
-    const int64_t v0 = __ldg(vbase + p), v1 = __ldg(vbase + p + 1);
-    const float p0 = 1.0f / (float)(v1 - v0);
-    const float added = (1.0f - damping) * p0;
-    const int64_t first = v0 + (int64_t)rank * kPartThreads + threadIdx.x;
-    for (int64_t v = first; v < v1; v += stride) {
-      const int deg = __ldg(g.out.off + v + 1) - __ldg(g.out.off + v);
-      pc[v] = p0;
-      pn[v] = 0.0f;
-      c0[v] = deg > 0 ? p0 / (float)deg : 0.0f;
-    }
-    cluster.sync();
-    float *A = pc, *B = pn, *cc = c0, *cn = c1;
-    for (int it = 0; it < iters; ++it) {
-      for (int64_t v = first; v < v1; v += stride) {
-        const int e0 = __ldg(g.in.off + v), e1 = __ldg(g.in.off + v + 1);
-        float acc = -0.0f;
-        int e = e0;
-        for (; e + 3 < e1; e += 4) {
-          const int s0 = __ldg(g.in.idx + e), s1 = __ldg(g.in.idx + e + 1);
-          const int s2 = __ldg(g.in.idx + e + 2), s3 = __ldg(g.in.idx + e + 3);
-          acc += (cc[s0] + cc[s1]) + (cc[s2] + cc[s3]);
-        }
-        for (; e < e1; ++e) acc += cc[__ldg(g.in.idx + e)];
-        const bool in_f = !signbit(cc[v]);
-        const bool hit = !signbit(acc);
-        float nb = B[v] + acc;
-        if (in_f) {
-          nb = damping * nb + added;
-          A[v] = 0.0f;
-        }
-        B[v] = nb;
-        const int deg = __ldg(g.out.off + v + 1) - __ldg(g.out.off + v);
-        cn[v] = hit ? (deg > 0 ? nb / (float)deg : 0.0f) : -0.0f;
-      }
-      cluster.sync();
-      float *t = A; A = B; B = t;
-      t = cc; cc = cn; cn = t;
-    }
-    for (int64_t v = first; v < v1; v += stride) out[v] = A[v];
-    cluster.sync();
-  }
-}
-
-void run_pagerank_parts(pm_graph *g, int iters, double damping, float *d_out) {
-  Engine &E = g->E;
-  const int64_t n = g->n;
-  const int count = (int)g->parts.size() - 1;
-  float *pc = (float *)g->scratch_buf(0, (size_t)n * 4);
-  float *pn = (float *)g->scratch_buf(1, (size_t)n * 4);
-  float *c0 = (float *)g->scratch_buf(2, (size_t)n * 4);
-  float *c1 = (float *)g->scratch_buf(3, (size_t)n * 4);
-  static const int clusters = [] {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kPartCluster * 64);
-    cfg.blockDim = dim3(kPartThreads);
-    int r = 0;
-    PM_CUDA(cudaOccupancyMaxActiveClusters(&r, (void *)k_pagerank_parts, &cfg));
-    return std::max(r, 1);
-  }();
-  const int grid = kPartCluster * std::max(1, std::min(clusters, count));
-  PM_CUDA(cudaMemsetAsync(E.d_cnt, 0, sizeof(Counters), E.stream));
-  E.prof.begin("pagerank_parts", E.stream);
-  PM_LAUNCH(k_pagerank_parts, grid, kPartThreads, 0, E.stream, E.g, g->parts_vbase.as<int64_t>(),
-            g->parts_order.as<int32_t>(), count, iters, (float)damping, pc, pn, c0, c1, d_out, E.d_cnt);
-  E.prof.end(E.stream);
 }
 
 }  // namespace pm

@@ -567,6 +567,7 @@ void set_parts(pm_graph *g, const std::vector<int64_t> &vbase) {
   PM_CUDA(cudaMemcpyAsync(g->parts_order.p, order.data(), count * 4, cudaMemcpyHostToDevice, g->E.stream));
   PM_CUDA(cudaStreamSynchronize(g->E.stream));
   g->parts = vbase;
+  g->parts_layout = PartsLayout{};
 }
 
 void gen_weights(pm_graph *g, uint64_t seed, int32_t wmax, bool is_float) {
