@@ -635,8 +635,8 @@ template <class T>
 bool run_pagerank_sorted(pm_graph *g, int iters, double damping, T *d_out, double *d_resid);
 
 // Whole graphs sum over the degree-sorted copy (pm_sorted.cu); a partition,
-// whose ranks exchange ranges of vertices, and a handle without room for the
-// copy pull over the CSC.
+// whose ranks exchange ranges of vertices, a handle without room for the copy
+// and a damping outside [0, 1] pull over the CSC.
 template <class T>
 void run_pagerank(pm_graph *g, int iters, double damping, T *d_out, double *d_resid) {
   if (run_pagerank_sorted<T>(g, iters, damping, d_out, d_resid)) return;

@@ -371,7 +371,9 @@ template <class T>
 bool run_pagerank_sorted(pm_graph *g, int iters, double damping, T *d_out, double *d_resid) {
   Engine &E = g->E;
   SortedView a;
-  if (!ensure_sorted(g, false, false, a)) return false;
+  // outside [0, 1] a rank may turn negative: the sign of a contribution is then
+  // no longer the frontier alone, and a vertex can come back into it
+  if (!(damping >= 0.0 && damping <= 1.0) || !ensure_sorted(g, false, false, a)) return false;
   const int64_t n = g->n;
   T *c0 = (T *)g->scratch_buf(0, (size_t)n * sizeof(T));
   T *c1 = (T *)g->scratch_buf(1, (size_t)n * sizeof(T));
@@ -386,7 +388,7 @@ bool run_pagerank_sorted(pm_graph *g, int iters, double damping, T *d_out, doubl
   auto gone = [&](int t) { return (iters - 1 - t) % 2 == 0 ? added : T(0); };
   PM_LAUNCH((k_prs_init<T>), E.grid_for(n, 256, 16), 256, 0, E.stream, c0, c1, p, a.odeg, n, (int64_t)a.rl,
             iters > 0 ? gone(0) : p0);
-  E.run_loop(loop_key("pagerank_sorted", (int)sizeof(T), iters, damping, c0, c1, p, d_resid), [&] {
+  E.run_loop(loop_key("pagerank_sorted", (int)sizeof(T), iters, damping, c0, c1, p, aux, d_resid), [&] {
     T *x = c0, *y = c1;
     for (int it = 0; it < iters; ++it) {
       E.prof.begin("pagerank", E.stream);
@@ -443,7 +445,7 @@ bool run_spmv_sorted(pm_graph *g, const T *d_x0, int iters, T *d_y, double *d_no
   }
   launch_to_positions(E, a, d_x0, x);
   launch_fill_tail(E, a, y, T(0));
-  E.run_loop(loop_key("spmv_sorted", (int)sizeof(T), iters, x, y, (const void *)a.w, d_norm), [&] {
+  E.run_loop(loop_key("spmv_sorted", (int)sizeof(T), iters, x, y, (const void *)a.w, aux, d_norm), [&] {
     T *s = x, *t = y;
     for (int it = 0; it < iters; ++it) {
       E.prof.begin("spmv", E.stream);
