@@ -153,6 +153,7 @@ struct pm_graph : pm::IdleFreeBase {
   std::vector<int64_t> parts;       // count+1 vertex offsets (host copy); empty if none
   pm::DevBuf parts_vbase, parts_order;
   pm::PartsLayout parts_layout;
+  bool lean = false;  // the call runs again after running out of memory: no copies
   // 1D vertex partition across processes (pm_graph_create_partition): this
   // handle holds the edges whose destination lies in [part_lo, part_hi)
   // (rank r owns [part_bounds[r], part_bounds[r+1]); part_wbounds are the
@@ -195,6 +196,7 @@ namespace pm {
 // Builds every derived structure (CSC, groups, heavy chunks, workspaces)
 // once out.off / out.idx hold a validated CSR on the device.
 void finish_graph(pm_graph *g);
+bool drop_copies(pm_graph *g);
 // Rebuilds what depends on E.tune (heavy tables when heavy_deg changed from
 // old_heavy_deg, the views, the partials) and drops captured loops.
 void apply_tunables(pm_graph *g, int32_t old_heavy_deg);

@@ -88,12 +88,28 @@ struct NvtxRange {
   NvtxRange &operator=(const NvtxRange &) = delete;
 };
 
+static thread_local pm_graph *t_entered = nullptr;  // the handle of this thread's call (enter)
+
 template <class Fn>
 static pm_status guard(const char *name, Fn &&fn) {
   NvtxRange range(name);
   AllocScope scope(AllocCtx{});  // enter() names the call's stream
+  t_entered = nullptr;
   try {
-    fn();
+    try {
+      fn();
+    } catch (const Failure &f) {
+      // Out of memory: without the copies that only make calls faster there
+      // may be room (every call has a form that does without them).
+      pm_graph *g = t_entered;
+      if (f.status != PM_ERR_OOM || !g || !drop_copies(g)) throw;
+      struct Lean {
+        pm_graph *g;
+        explicit Lean(pm_graph *h) : g(h) { g->lean = true; }
+        ~Lean() { g->lean = false; }
+      } lean(g);
+      fn();
+    }
     t_last_error.clear();
     return PM_OK;
   } catch (const Failure &f) {
@@ -181,6 +197,7 @@ static void enter(pm_graph *g) {
   need(g != nullptr, "null graph handle");
   PM_CUDA(cudaSetDevice(g->device));
   set_alloc_ctx(AllocCtx{g->E.stream, false});  // this call's buffers live in this stream's order
+  t_entered = g;
 }
 
 extern "C" {

@@ -115,6 +115,7 @@ __global__ void k_parts_fill(GraphView g, PartsView a, int64_t npos, const int32
 // there is no memory for it: k_pagerank_parts then runs in vertex order.
 static bool ensure_parts_layout(pm_graph *g) {
   PartsLayout &L = g->parts_layout;
+  if (g->lean) return false;
   if (L.state != 0) return L.state > 0;
   Engine &E = g->E;
   cudaStream_t st = E.stream;

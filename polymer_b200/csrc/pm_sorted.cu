@@ -245,7 +245,7 @@ static void build_sorted(pm_graph *g, bool csr, SortedAdj &b) {
 
 const SortedView *ensure_sorted(pm_graph *g, bool csr, bool weighted, SortedView &view) {
   // slices pad by at most 32 * kSortShort slots in all, and round up once
-  if (g->is_part || g->m > (1ll << 31) - 8192) return nullptr;
+  if (g->is_part || g->lean || g->m > (1ll << 31) - 8192) return nullptr;
   SortedAdj &b = csr ? g->sorted_out : g->sorted_in;
   Engine &E = g->E;
   try {
@@ -268,6 +268,18 @@ const SortedView *ensure_sorted(pm_graph *g, bool csr, bool weighted, SortedView
   view = *b.view;
   view.w = weighted ? b.w.as<float>() : nullptr;
   return &view;
+}
+
+// Gives the copies' memory back (and the captured loops that read them); false
+// when there was nothing to give.
+bool drop_copies(pm_graph *g) {
+  if (!g->sorted_in.odeg.p && !g->sorted_out.odeg.p && g->parts_layout.state <= 0) return false;
+  PM_CUDA(cudaStreamSynchronize(g->E.stream));
+  g->E.release_graphs();
+  g->sorted_in = SortedAdj{};
+  g->sorted_out = SortedAdj{};
+  if (g->parts_layout.state > 0) g->parts_layout = PartsLayout{};
+  return true;
 }
 
 __global__ void __launch_bounds__(kAuxSlots) k_fix_end(double2 *aux, double tail_first, double tail_norm,
