@@ -1,6 +1,6 @@
-// pm_batch.cu -- batched workloads: multi-source BellmanFord (64 int32
-// distance lanes per vertex) and personalised PageRank for up to 32 seeds
-// (multi-source BFS: pm_msbfs.cu; the parts of a disjoint union: pm_parts.cu).
+// pm_batch.cu -- batched workloads: multi-source BellmanFord, 64 int32
+// distance lanes per vertex (personalised PageRank: pm_ppr.cu; multi-source
+// BFS: pm_msbfs.cu; the parts of a disjoint union: pm_parts.cu).
 #include <cub/cub.cuh>
 
 #include "pm_sorted.cuh"
@@ -415,240 +415,6 @@ void run_bf_multi(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_dist_
   PM_LAUNCH(k_bf_multi_transpose, tg, tb, 0, E.stream, dist, n, k, d_dist_out, E.d_cnt + 2);
   s.reached = (int64_t)E.read_counters()[2].size;
   if (st) *st = s;
-}
-
-// ===========================================================================
-// Personalised PageRank for up to 32 seeds in one SpMM-shaped pull per
-// iteration (PR_F's push p[s]/outdeg(s) and PR_Vertex_F's damping,
-// numa-PageRank.C:87-90, 125-137, applied to all vectors at once, teleport to
-// each vector's seed).  The contribution matrix C (n x COLS floats, row-major,
-// C[u][j] = x_j[u] / outdeg(u); COLS the seeds rounded up to 8, 16 or 32) is
-// gathered one row per in-edge, COLS / 4 lanes holding a float4 each.  Rows
-// are taken in order of in-degree (pm_sorted.cu): the longest by a warp each,
-// the others COLS / 4 lanes each, so that the rows of a warp have the same
-// length and a sum needs no shuffles; a vertex without in-edges never changes
-// after the first iteration and is written once.  Rows with more than
-// g.heavy_deg in-edges are summed by chunk CTAs first.
-//
-// What bounds it: the loads in flight for the row gathers and the instructions
-// around them.  A warp per row in vertex order spent 61 % of the issue slots
-// at 23 % of the L2's rate.  32 seeds, 20 iterations, directed 2^24-vertex,
-// 263 M-edge R-MAT: 108 ms with a lane per column, 101.7 with four rows per
-// load, 87.8 in this form with four CTAs per SM (62 registers), 78.7 with six
-// and 73.9 ms with eight (32 registers): warps hide the gathers better than
-// registers do.
-// ===========================================================================
-constexpr int kPprCols = 32;
-
-__device__ __forceinline__ void add4(float4 &a, const float4 &b) {
-  a.x += b.x;
-  a.y += b.y;
-  a.z += b.z;
-  a.w += b.w;
-}
-template <int COLS>
-__device__ __forceinline__ float4 xor_add4(float4 a) {  // over the groups of COLS / 4 lanes of a warp
-#pragma unroll
-  for (int d = COLS / 4; d < 32; d <<= 1) {
-    a.x += __shfl_xor_sync(0xffffffffu, a.x, d);
-    a.y += __shfl_xor_sync(0xffffffffu, a.y, d);
-    a.z += __shfl_xor_sync(0xffffffffu, a.z, d);
-    a.w += __shfl_xor_sync(0xffffffffu, a.w, d);
-  }
-  return a;
-}
-
-// This lane group's sum of the rows named by idx[e], idx[e + step], ... below
-// e1 (the lane's four columns): eight row gathers in flight per group.  All
-// lanes of the warp call it; groups may have different rows and lengths.
-template <int COLS>
-__device__ __forceinline__ float4 ppr_sum(const int32_t *__restrict__ idx, int e, int e1, int step,
-                                          const float *__restrict__ c) {
-  constexpr int L = COLS / 4, U = 8, I = U / L;  // lanes per row; edges and id loads per step
-  const int sub = lane_id() % L;
-  const float *col = c + 4 * sub;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  while (__any_sync(0xffffffffu, e < e1)) {
-    int id[I];
-#pragma unroll
-    for (int i = 0; i < I; ++i) {
-      const int x = e + (i * L + sub) * step;
-      id[i] = x < e1 ? __ldcs(idx + x) : -1;
-    }
-    float4 v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int s = __shfl_sync(0xffffffffu, id[u / L], u % L, L);
-      v[u] = s >= 0 ? __ldg(reinterpret_cast<const float4 *>(col + (int64_t)s * COLS)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) add4(acc, v[u]);
-    e += U * step;
-  }
-  return acc;
-}
-
-template <int COLS>
-__global__ void __launch_bounds__(256) k_ppr_heavy(GraphView g, const float *__restrict__ c,
-                                                   float *__restrict__ partials) {
-  constexpr int L = COLS / 4;
-  __shared__ float4 s_part[8][L];
-  const int ch = blockIdx.x;
-  if (ch >= g.in.nchunks) return;
-  const int lane = lane_id(), wid = threadIdx.x >> 5;
-  const int r = __ldg(g.in.hrow + ch);
-  const int k = ch - __ldg(g.in.hfirst + r);
-  const int row_end = __ldg(g.in.off + r + 1);
-  const int e0 = __ldg(g.in.off + r) + k * kChunkEdges, e1 = min(row_end - e0, kChunkEdges) + e0;
-  const float4 sum = xor_add4<COLS>(ppr_sum<COLS>(g.in.idx, e0 + (int)threadIdx.x / L, e1, 256 / L, c));
-  if (lane < L) s_part[wid][lane] = sum;
-  __syncthreads();
-  if (wid == 0 && lane < L) {
-    float4 t = s_part[0][lane];
-    for (int w = 1; w < 8; ++w) add4(t, s_part[w][lane]);
-    reinterpret_cast<float4 *>(partials)[(int64_t)ch * L + lane] = t;
-  }
-}
-
-// Row v's new value and contribution: this lane's four columns.
-template <int COLS>
-__device__ __forceinline__ void ppr_commit(const GraphView &g, int v, const float4 &acc, const int4 &seed, float damping,
-                                           float *__restrict__ c_next, float *__restrict__ y_out, int k_out) {
-  const int sub = lane_id() % (COLS / 4);
-  const int od = __ldg(g.out.off + v + 1) - __ldg(g.out.off + v);
-  const float jump = 1.0f - damping;
-  float4 y;
-  y.x = damping * acc.x + (v == seed.x ? jump : 0.0f);
-  y.y = damping * acc.y + (v == seed.y ? jump : 0.0f);
-  y.z = damping * acc.z + (v == seed.z ? jump : 0.0f);
-  y.w = damping * acc.w + (v == seed.w ? jump : 0.0f);
-  if (y_out) {
-    float *out = y_out + (int64_t)v * k_out + 4 * sub;
-    if (4 * sub < k_out) out[0] = y.x;
-    if (4 * sub + 1 < k_out) out[1] = y.y;
-    if (4 * sub + 2 < k_out) out[2] = y.z;
-    if (4 * sub + 3 < k_out) out[3] = y.w;
-  }
-  const float f = (float)od;
-  const float4 cn = od > 0 ? make_float4(y.x / f, y.y / f, y.z / f, y.w / f) : make_float4(0.f, 0.f, 0.f, 0.f);
-  *reinterpret_cast<float4 *>(c_next + (int64_t)v * COLS + 4 * sub) = cn;
-}
-// The seeds of this lane's columns (-1 past the last).
-template <int COLS>
-__device__ __forceinline__ int4 ppr_seeds(const int32_t *__restrict__ seeds, int k) {
-  const int j = 4 * (lane_id() % (COLS / 4));
-  return make_int4(j < k ? __ldg(seeds + j) : -1, j + 1 < k ? __ldg(seeds + j + 1) : -1,
-                   j + 2 < k ? __ldg(seeds + j + 2) : -1, j + 3 < k ? __ldg(seeds + j + 3) : -1);
-}
-
-// order: vertices by in-degree; [0, rh) have kSortLong in-edges or more and
-// take a warp each, [rh, rl) a group of lanes each.
-template <int COLS>
-__global__ void __launch_bounds__(256, COLS == 32 ? 8 : 6) k_ppr_pull(GraphView g, const int32_t *__restrict__ order, int rh, int rl,
-                                                     const float *__restrict__ c_cur, float *__restrict__ c_next,
-                                                     float *__restrict__ y_out, int k_out,
-                                                     const float *__restrict__ partials,
-                                                     const int32_t *__restrict__ seeds, float damping) {
-  constexpr int L = COLS / 4;
-  const int lane = lane_id(), group = lane / L;
-  const int64_t t = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int4 seed = ppr_seeds<COLS>(seeds, k_out);
-  if (t < rh) {
-    const int v = __ldg(order + t);
-    const int o = __ldg(g.in.off + v), o1 = __ldg(g.in.off + v + 1);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (o1 - o > g.heavy_deg) {
-      const int first = __ldg(g.in.hfirst + v), nch = (o1 - o + kChunkEdges - 1) / kChunkEdges;
-      for (int q = 0; q < nch; ++q)
-        add4(acc, __ldg(reinterpret_cast<const float4 *>(partials) + (int64_t)(first + q) * L + lane % L));
-    } else {
-      acc = xor_add4<COLS>(ppr_sum<COLS>(g.in.idx, o + group, o1, 32 / L, c_cur));
-    }
-    if (lane < L) ppr_commit<COLS>(g, v, acc, seed, damping, c_next, y_out, k_out);
-  } else {
-    const int64_t r = rh + (t - rh) * (32 / L) + group;
-    int v = 0, o = 0, o1 = 0;
-    bool heavy = false;
-    if (r < rl) {
-      v = __ldg(order + r);
-      o = __ldg(g.in.off + v);
-      o1 = __ldg(g.in.off + v + 1);
-      heavy = o1 - o > g.heavy_deg;  // a cut-off below kSortLong
-    }
-    float4 acc = ppr_sum<COLS>(g.in.idx, heavy ? o1 : o, o1, 1, c_cur);
-    if (heavy) acc = __ldg(reinterpret_cast<const float4 *>(partials) + (int64_t)__ldg(g.in.hfirst + v) * L + lane % L);
-    if (r < rl) ppr_commit<COLS>(g, v, acc, seed, damping, c_next, y_out, k_out);
-  }
-}
-
-// The vertices without in-edges (order[rl .. n)): their rows of the second
-// matrix and of the result, which no iteration changes.
-template <int COLS>
-__global__ void __launch_bounds__(256) k_ppr_tail(GraphView g, const int32_t *__restrict__ order, int rl,
-                                                  float *__restrict__ c, float *__restrict__ y_out, int k_out,
-                                                  const int32_t *__restrict__ seeds, float damping) {
-  constexpr int L = COLS / 4;
-  const int4 seed = ppr_seeds<COLS>(seeds, k_out);
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x / L;
-  for (int64_t r = rl + ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L; r < g.n; r += stride)
-    ppr_commit<COLS>(g, __ldg(order + r), make_float4(0.f, 0.f, 0.f, 0.f), seed, damping, c, y_out, k_out);
-}
-
-// C0[v][j] = x / outdeg(v) for the seeds v = seeds[j]; with tail only those
-// without in-edges.
-__global__ void k_ppr_seed(const int32_t *seeds, int k, GraphView g, float *c, int cols, float x, bool tail,
-                           float *y0, int k_out) {
-  const int j = threadIdx.x;
-  if (j >= k) return;
-  const int v = seeds[j];
-  if (tail && g.in.off[v + 1] > g.in.off[v]) return;
-  const int od = g.out.off[v + 1] - g.out.off[v];
-  c[(int64_t)v * cols + j] = od > 0 ? x / (float)od : 0.f;
-  if (y0) y0[(int64_t)v * k_out + j] = x;
-}
-
-template <int COLS>
-static void run_ppr_cols(pm_graph *g, const int32_t *d_seeds, int k, int iters, double damping, float *d_out) {
-  Engine &E = g->E;
-  const int64_t n = g->n;
-  const RowOrder &o = ensure_row_order(g, false);
-  const int32_t *order = o.order.as<int32_t>();
-  const int rh = o.cuts[1], rl = o.cuts[3];
-  float *c0 = (float *)g->scratch_buf(0, (size_t)n * COLS * 4);
-  float *c1 = (float *)g->scratch_buf(1, (size_t)n * COLS * 4);
-  float *part = (float *)g->scratch_buf(2, (size_t)std::max(E.g.in.nchunks, 1) * COLS * 4);
-  const float dmp = (float)damping;
-  PM_CUDA(cudaMemsetAsync(c0, 0, (size_t)n * COLS * 4, E.stream));
-  if (iters == 0) PM_CUDA(cudaMemsetAsync(d_out, 0, (size_t)n * k * 4, E.stream));
-  PM_LAUNCH(k_ppr_seed, 1, 32, 0, E.stream, d_seeds, k, E.g, c0, COLS, 1.0f, false, iters == 0 ? d_out : nullptr, k);
-  if (iters > 0 && rl < n)
-    PM_LAUNCH((k_ppr_tail<COLS>), E.grid_for((n - rl) * (COLS / 4), 256, 8), 256, 0, E.stream, E.g, order, rl, c1,
-              d_out, k, d_seeds, dmp);
-  const int64_t warps = rh + ((int64_t)(rl - rh) * (COLS / 4) + 31) / 32;
-  E.run_loop(loop_key("ppr", iters, k, damping, c0, c1, part, (const void *)d_seeds, d_out), [&] {
-    float *a = c0, *b = c1;
-    for (int it = 0; it < iters; ++it) {
-      E.prof.begin("ppr", E.stream);
-      if (E.g.in.nchunks > 0)
-        PM_LAUNCH((k_ppr_heavy<COLS>), E.g.in.nchunks, 256, 0, E.stream, E.g, a, part);
-      if (warps > 0)
-        PM_LAUNCH((k_ppr_pull<COLS>), (unsigned)((warps + 7) / 8), 256, 0, E.stream, E.g, order, rh, rl, a, b,
-                  it == iters - 1 ? d_out : nullptr, k, part, d_seeds, dmp);
-      // the seeds without in-edges settle in the first matrix, too
-      if (it == 0) PM_LAUNCH(k_ppr_seed, 1, 32, 0, E.stream, d_seeds, k, E.g, a, COLS, 1.0f - dmp, true, nullptr, k);
-      E.prof.end(E.stream);
-      std::swap(a, b);
-    }
-  });
-}
-
-void run_ppr(pm_graph *g, const int32_t *d_seeds, int k, int iters, double damping, float *d_out) {
-  if (k <= 8)
-    run_ppr_cols<8>(g, d_seeds, k, iters, damping, d_out);
-  else if (k <= 16)
-    run_ppr_cols<16>(g, d_seeds, k, iters, damping, d_out);
-  else
-    run_ppr_cols<kPprCols>(g, d_seeds, k, iters, damping, d_out);
 }
 
 }  // namespace pm
