@@ -16,9 +16,9 @@ using u64 = unsigned long long;
 // active[v] has bit l set when lane l of v fell in the last round.  A round
 // follows BF's direction rule on the union frontier (|F| + outdeg(F) >=
 // threshold is dense):
-//  * dense: a warp owns a CSC row, thread t owns lanes t and t+32; for each
-//    in-edge whose source has active lanes it gathers the source's row and
-//    relaxes those lanes; the row's new active word is written in full;
+//  * dense: eight lanes of a warp (or, for long rows, all) own a CSC row; for
+//    each in-edge whose source has active lanes they gather the source's row
+//    and take its minimum with the weight added;
 //  * sparse: the frontier's out-edges are cut into 32-edge chunks (a scan of
 //    the queued out-degrees); for each edge the warp relaxes the active lanes
 //    of the target with atomicMin and ORs the lanes that fell into the
@@ -26,51 +26,91 @@ using u64 = unsigned long long;
 // Distances only fall, so reading a row another warp is lowering in the same
 // round is harmless: the lower value is a real path length and the lane that
 // fell is in the next frontier either way.
+//
+// What bounds it: the instructions around the pull's row gathers (72 % of the
+// issue slots at 22 % of the L2's rate with half a warp per row and a test per
+// lane; a load, two shuffles and eight add-and-minimum instructions per four
+// rows now).  50 sources, 1.5 M vertices, 42 M edges: 9.0 ms with a warp per
+// row in vertex order, 6.65 with half a warp per row by in-degree, 4.33 here
+// (a dense round 1.25 -> 0.78 ms).
 // ===========================================================================
 constexpr int kLanes = 64;
-constexpr int kBfUnroll = 4;      // pull: in-edges whose row gathers are in flight together per half-warp
-// Resident CTAs per SM of the pull: 50 sources on a 1.5 M-vertex, 42 M-edge
-// R-MAT take 8.37 ms with four (58 registers), 7.11 with five, 6.64 with six
-// (40 registers) and 6.75 with eight; a warp per row in vertex order, two
-// 128-byte loads a row, took 8.87 to 9.16.
-constexpr int kBfCtas = 6;
+// Resident CTAs per SM of the pull: with eight, a row in flight per group of
+// lanes, 50 sources on a 1.5 M-vertex, 42 M-edge R-MAT take 4.33 ms; with six
+// and two rows in flight 4.44, with five and three 4.72, with four and four
+// 4.82.
+constexpr int kBfCtas = 8;
 constexpr int kBfPushUnroll = 2;  // push: out-edges whose target rows are read together per warp
 
 // active -> queue of frontier vertices with out-edges (and their degrees);
-// c->size = |F|, c->edges = outdeg(F), c->aux = queue length.
-__global__ void k_bf_multi_frontier(const u64 *__restrict__ active, const int32_t *__restrict__ out_off,
-                                    int64_t n, int32_t *__restrict__ queue, int32_t *__restrict__ qdeg,
-                                    Counters *c) {
-  const int lane = lane_id();
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+// c->size = |F|, c->edges = outdeg(F), c->aux = queue length.  A block takes
+// 1024 vertices at a time, four side by side per thread, and reserves their
+// queue slots with one atomic (an atomic per warp and 32 vertices took 60 us
+// for a frontier of most of 1.5 M vertices).
+__global__ void __launch_bounds__(256) k_bf_multi_frontier(const u64 *__restrict__ active,
+                                                           const int32_t *__restrict__ out_off, int64_t n,
+                                                           int32_t *__restrict__ queue, int32_t *__restrict__ qdeg,
+                                                           Counters *c) {
+  __shared__ unsigned s_count[8];
+  __shared__ unsigned long long s_at, s_size[8], s_edges[8];
+  const int lane = lane_id(), wid = threadIdx.x >> 5;
+  constexpr int U = 4;
   unsigned long long size = 0, edges = 0;
-  for (int64_t base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; base < n;
-       base += warps * 32) {
-    const int64_t v = base + lane;
-    int deg = 0;
-    bool act = false;
-    if (v < n) {
-      act = active[v] != 0ull;
-      if (act) deg = __ldg(out_off + v + 1) - __ldg(out_off + v);
+  for (int64_t base = (int64_t)blockIdx.x * (256 * U); base < n; base += (int64_t)gridDim.x * (256 * U)) {
+    bool act[U];
+    int deg[U];
+    unsigned push[U];
+    int count = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t v = base + u * 256 + threadIdx.x;
+      act[u] = v < n && active[v] != 0ull;
     }
-    size += act;
-    edges += (unsigned)deg;
-    const unsigned push = __ballot_sync(0xffffffffu, deg > 0);
-    if (push) {
-      unsigned long long pos = 0;
-      if (lane == 0) pos = atomicAdd(&c->aux, (unsigned long long)__popc(push));
-      pos = shfl_idx(pos, 0) + __popc(push & ((1u << lane) - 1u));
-      if (deg > 0) {
-        queue[pos] = (int32_t)v;
-        qdeg[pos] = deg;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t v = base + u * 256 + threadIdx.x;
+      deg[u] = act[u] ? __ldg(out_off + v + 1) - __ldg(out_off + v) : 0;
+      size += act[u];
+      edges += (unsigned)deg[u];
+      push[u] = __ballot_sync(0xffffffffu, deg[u] > 0);
+      count += __popc(push[u]);
+    }
+    if (lane == 0) s_count[wid] = (unsigned)count;
+    __syncthreads();
+    unsigned before = 0, all = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      before += i < wid ? s_count[i] : 0u;
+      all += s_count[i];
+    }
+    if (threadIdx.x == 0 && all) s_at = atomicAdd(&c->aux, (unsigned long long)all);
+    __syncthreads();
+    unsigned long long pos = s_at + before;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (deg[u] > 0) {
+        const unsigned long long at = pos + __popc(push[u] & ((1u << lane) - 1u));
+        queue[at] = (int32_t)(base + u * 256 + threadIdx.x);
+        qdeg[at] = deg[u];
       }
+      pos += __popc(push[u]);
     }
+    __syncthreads();  // s_count and s_at are free again
   }
   size = warp_sum(size);
   edges = warp_sum(edges);
-  if (lane == 0 && size) {
-    atomicAdd(&c->size, size);
-    atomicAdd(&c->edges, edges);
+  if (lane == 0) {
+    s_size[wid] = size;
+    s_edges[wid] = edges;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; ++i) {
+      size += s_size[i];
+      edges += s_edges[i];
+    }
+    if (size) atomicAdd(&c->size, size);
+    if (edges) atomicAdd(&c->edges, edges);
   }
 }
 
@@ -159,75 +199,77 @@ __global__ void __launch_bounds__(256) k_bf_multi_push(const int32_t *__restrict
   }
 }
 
-// The least dist[s] + w over this half-warp's in-edges whose sources have
-// active lanes: 16 edges from e on, then from e + step on, ... below e1.  Half
-// a warp holds a source's row (int4: lanes 4 t .. 4 t + 3 of the 64 on its
-// thread t), so one load brings a row to each half and a step has kBfUnroll
-// rows per half in flight.  All lanes of the warp call it; the halves may have
-// different rows and lengths.
-__device__ __forceinline__ int4 bf_multi_relax(const int32_t *__restrict__ in_idx, const int32_t *__restrict__ w_in,
-                                               const int32_t *dist, const u64 *__restrict__ active, int e, int e1,
-                                               int step) {
-  const int t = lane_id() & 15, quad = t * 4, shift = lane_id() & 16;
-  int4 m = make_int4(kDevBFInf, kDevBFInf, kDevBFInf, kDevBFInf);
+// Eight of a row's 64 distances: 32 bytes, one load.
+struct Oct {
+  int32_t x[8];
+};
+__device__ __forceinline__ Oct ld_oct(const int32_t *p) {
+  Oct v;
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]), "=r"(v.x[4]), "=r"(v.x[5]), "=r"(v.x[6]),
+                 "=r"(v.x[7])
+               : "l"(p));
+  return v;
+}
+
+constexpr int kBfSub = 8;  // lanes per row
+constexpr int kBfSmallWeight = 1 << 30;
+
+// The least dist[s] + w over this group's in-edges whose sources have active
+// lanes: kBfSub edges from e on, then from e + step on, ... below e1.  Eight
+// lanes hold a source's row (thread t lanes 8 t .. 8 t + 7), so that one load
+// instruction brings four rows.  A lane of such a source that is not active is
+// relaxed too: its distance, when finite, is a path's length that was pushed
+// when it fell, and pushing it again changes nothing.  An infinite one must
+// not be pushed over a negative weight, nor where the sum would wrap: a batch
+// with such a weight tests each value.  self: the group's own row, named by
+// the places without an edge.  All lanes of the warp call it; the groups may
+// have different rows and lengths.  col: dist at this thread's lanes.
+__device__ __forceinline__ Oct bf_multi_relax(const int32_t *__restrict__ in_idx, const int32_t *__restrict__ w_in,
+                                              const int32_t *col, const u64 *__restrict__ active, int self, int e,
+                                              int e1, int step) {
+  const int t = lane_id() & 7, shift = lane_id() & 24;
+  Oct m;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) m.x[i] = kDevBFInf;
   for (; __any_sync(0xffffffffu, e < e1); e += step) {
-    int s = 0;
-    u64 act = 0;
+    int s = self;
+    bool act = false;
     int32_t w = 0;
     if (e + t < e1) {
       s = __ldcs(in_idx + e + t);
-      act = __ldg(active + s);
+      act = __ldg(active + s) != 0ull;
       w = __ldcs(w_in + e + t);
     }
-    unsigned todo = (__ballot_sync(0xffffffffu, act != 0) >> shift) & 0xffffu;
+    unsigned todo = (__ballot_sync(0xffffffffu, act) >> shift) & 0xffu;
+    const bool plain = __all_sync(0xffffffffu, (unsigned)w <= (unsigned)kBfSmallWeight);
+    int j = 0;  // a group that is done repeats its last edge (or place)
     while (__any_sync(0xffffffffu, todo != 0u)) {
-      int4 v[kBfUnroll];
-      unsigned on[kBfUnroll];
-      int32_t wj[kBfUnroll];
+      if (todo) j = __ffs(todo) - 1;
+      todo &= todo - 1u;
+      const int sj = __shfl_sync(0xffffffffu, s, j, 8);
+      const int32_t wj = __shfl_sync(0xffffffffu, w, j, 8);
+      const Oct v = ld_oct(col + (int64_t)sj * kLanes);
+      if (plain) {
 #pragma unroll
-      for (int u = 0; u < kBfUnroll; ++u) {
-        const int j = todo ? __ffs(todo) - 1 : 0;
-        const bool take = todo != 0u;
-        todo &= todo - 1u;
-        const int sj = __shfl_sync(0xffffffffu, s, j, 16);
-        const unsigned lo = __shfl_sync(0xffffffffu, (unsigned)act, j, 16),
-                       hi = __shfl_sync(0xffffffffu, (unsigned)(act >> 32), j, 16);
-        wj[u] = __shfl_sync(0xffffffffu, w, j, 16);
-        on[u] = take ? ((quad < 32 ? lo >> quad : hi >> (quad - 32)) & 15u) : 0u;
-        v[u] = make_int4(0, 0, 0, 0);
-        if (on[u]) v[u] = *reinterpret_cast<const int4 *>(dist + (int64_t)sj * kLanes + quad);
-      }
+        for (int i = 0; i < 8; ++i) m.x[i] = __viaddmin_s32(v.x[i], wj, m.x[i]);
+      } else {
 #pragma unroll
-      for (int u = 0; u < kBfUnroll; ++u) {
-        if (on[u] & 1u) m.x = min(m.x, v[u].x + wj[u]);
-        if (on[u] & 2u) m.y = min(m.y, v[u].y + wj[u]);
-        if (on[u] & 4u) m.z = min(m.z, v[u].z + wj[u]);
-        if (on[u] & 8u) m.w = min(m.w, v[u].w + wj[u]);
+        for (int i = 0; i < 8; ++i)
+          if (v.x[i] < kDevBFInf) m.x[i] = min(m.x[i], v.x[i] + wj);
       }
     }
   }
   return m;
 }
-// Both halves' minima of one row, on both.
-__device__ __forceinline__ int4 bf_multi_join(int4 m) {
-  m.x = min(m.x, __shfl_xor_sync(0xffffffffu, m.x, 16));
-  m.y = min(m.y, __shfl_xor_sync(0xffffffffu, m.y, 16));
-  m.z = min(m.z, __shfl_xor_sync(0xffffffffu, m.z, 16));
-  m.w = min(m.w, __shfl_xor_sync(0xffffffffu, m.w, 16));
-  return m;
-}
-
-// The 64-bit mask whose bits 4 t .. 4 t + 3 are the nibble of the half's
-// thread t, on every lane of that half.
-__device__ __forceinline__ u64 bf_multi_mask(unsigned nibble) {
-  const int t = lane_id() & 15;
-  unsigned lo = t < 8 ? nibble << (4 * t) : 0u, hi = t < 8 ? 0u : nibble << (4 * (t - 8));
+// The four groups' minima of one row, on all of them.
+__device__ __forceinline__ Oct bf_multi_join(Oct m) {
 #pragma unroll
-  for (int d = 8; d > 0; d >>= 1) {
-    lo |= __shfl_xor_sync(0xffffffffu, lo, d);
-    hi |= __shfl_xor_sync(0xffffffffu, hi, d);
+  for (int i = 0; i < 8; ++i) {
+    m.x[i] = min(m.x[i], __shfl_xor_sync(0xffffffffu, m.x[i], 8));
+    m.x[i] = min(m.x[i], __shfl_xor_sync(0xffffffffu, m.x[i], 16));
   }
-  return (u64)lo | ((u64)hi << 32);
+  return m;
 }
 
 constexpr int kBfPiece = 512;  // in-edges of one warp's piece of a heavy row
@@ -235,14 +277,18 @@ constexpr int kBfPiece = 512;  // in-edges of one warp's piece of a heavy row
 // Dense round, a warp per item: 512-edge pieces of the heavy rows (in-degree >
 // g.heavy_deg; they lower the row with atomicMin and OR the fallen lanes into
 // next_active, which starts at zero), then the light rows in order of
-// in-degree (order: pm_sorted.cu), a warp for each of [0, rh) and half a warp
+// in-degree (order: pm_sorted.cu), a warp for each of [0, rh) and kBfSub lanes
 // for each of [rh, rl).  A light row is relaxed in full by its lanes, which
-// write its next_active word.
+// write its next_active bytes.
 __global__ void __launch_bounds__(256, kBfCtas) k_bf_multi_pull(GraphView g, const int32_t *__restrict__ w_in,
                                                                 int32_t *dist, const u64 *__restrict__ active,
                                                                 u64 *next_active, int64_t heavy_pieces,
-                                                                const int32_t *__restrict__ order, int rh, int rl) {
-  const int lane = lane_id(), half = lane >> 4, t = lane & 15;
+                                                                const int32_t *__restrict__ order, int rh, int rl,
+                                                                int k) {
+  const int lane = lane_id(), group = lane / kBfSub, t = lane % kBfSub;
+  // threads past the k sources read thread 0's lanes (no further sector) and write nothing
+  const bool used = 8 * t < k;
+  const int32_t *col = dist + (used ? 8 * t : 0);
   int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (item < heavy_pieces) {
     const int c = (int)(item / (kChunkEdges / kBfPiece));
@@ -253,23 +299,19 @@ __global__ void __launch_bounds__(256, kBfCtas) k_bf_multi_pull(GraphView g, con
                           (int64_t)piece * kBfPiece;
     if (first >= row_end) return;
     const int e0 = (int)first, e1 = min(row_end - e0, kBfPiece) + e0;
-    const int4 m = bf_multi_join(bf_multi_relax(g.in.idx, w_in, dist, active, e0 + 16 * half, e1, 32));
+    const Oct m = bf_multi_join(bf_multi_relax(g.in.idx, w_in, col, active, r, e0 + kBfSub * group, e1, 32));
+    if (group != 0 || !used) return;
     unsigned fell = 0;
-    if (half == 0) {
-      int32_t *p = dist + (int64_t)r * kLanes + 4 * t;
-      const volatile int32_t *seen = p;
-      if (m.x < seen[0] && m.x < atomicMin(p, m.x)) fell |= 1u;
-      if (m.y < seen[1] && m.y < atomicMin(p + 1, m.y)) fell |= 2u;
-      if (m.z < seen[2] && m.z < atomicMin(p + 2, m.z)) fell |= 4u;
-      if (m.w < seen[3] && m.w < atomicMin(p + 3, m.w)) fell |= 8u;
-    }
-    const u64 mask = bf_multi_mask(fell);
-    if (lane == 0 && mask) atomicOr(next_active + r, mask);
+    int32_t *p = dist + (int64_t)r * kLanes + 8 * t;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (m.x[i] < *(const volatile int32_t *)(p + i) && m.x[i] < atomicMin(p + i, m.x[i])) fell |= 1u << i;
+    if (fell) atomicOr(reinterpret_cast<unsigned *>(next_active + r) + t / 4, fell << 8 * (t % 4));
     return;
   }
   item -= heavy_pieces;
   const bool whole = item < rh;  // the same for the whole warp
-  const int64_t r = whole ? item : rh + 2 * (item - rh) + half;
+  const int64_t r = whole ? item : rh + (32 / kBfSub) * (item - rh) + group;
   int v = 0, e0 = 0, e1 = 0;
   bool mine = r < rl;
   if (mine) {
@@ -280,15 +322,17 @@ __global__ void __launch_bounds__(256, kBfCtas) k_bf_multi_pull(GraphView g, con
     if (!mine) e1 = e0;
   }
   if (!__any_sync(0xffffffffu, mine)) return;
-  int4 *row = reinterpret_cast<int4 *>(dist + (int64_t)v * kLanes) + t;
-  const int4 old = *row;
-  int4 m = bf_multi_relax(g.in.idx, w_in, dist, active, whole ? e0 + 16 * half : e0, e1, whole ? 32 : 16);
+  Oct m = bf_multi_relax(g.in.idx, w_in, col, active, v, whole ? e0 + kBfSub * group : e0, e1, whole ? 32 : kBfSub);
   if (whole) m = bf_multi_join(m);
-  const unsigned fell = !mine ? 0u : (m.x < old.x) | (m.y < old.y) << 1 | (m.z < old.z) << 2 | (m.w < old.w) << 3;
-  const bool write = !whole || half == 0;
-  if (write && fell) *row = make_int4(min(m.x, old.x), min(m.y, old.y), min(m.z, old.z), min(m.w, old.w));
-  const u64 mask = bf_multi_mask(fell);
-  if (mine && write && t == 0 && mask) next_active[v] = mask;
+  if (!mine || !used || (whole && group != 0)) return;
+  int4 *row = reinterpret_cast<int4 *>(dist + (int64_t)v * kLanes) + 2 * t;
+  const int4 a = row[0], b = row[1];
+  const unsigned fell = (m.x[0] < a.x) | (m.x[1] < a.y) << 1 | (m.x[2] < a.z) << 2 | (m.x[3] < a.w) << 3 |
+                        (m.x[4] < b.x) << 4 | (m.x[5] < b.y) << 5 | (m.x[6] < b.z) << 6 | (m.x[7] < b.w) << 7;
+  if (!fell) return;
+  row[0] = make_int4(min(m.x[0], a.x), min(m.x[1], a.y), min(m.x[2], a.z), min(m.x[3], a.w));
+  row[1] = make_int4(min(m.x[4], b.x), min(m.x[5], b.y), min(m.x[6], b.z), min(m.x[7], b.w));
+  reinterpret_cast<uint8_t *>(next_active + v)[t] = (uint8_t)fell;
 }
 
 __global__ void k_bf_multi_init(int32_t *dist, u64 *active, int64_t n) {
@@ -374,14 +418,14 @@ void run_bf_multi(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_dist_
   const int64_t heavy_pieces = (int64_t)E.g.in.nchunks * (kChunkEdges / kBfPiece);
   const RowOrder &o = ensure_row_order(g, false);
   const int rh = o.cuts[1], rl = o.cuts[3];
-  const int64_t items = heavy_pieces + rh + (rl - rh + 1) / 2;
+  const int64_t items = heavy_pieces + rh + ((int64_t)(rl - rh) * kBfSub + 31) / 32;
   const unsigned pull_grid = (unsigned)((items + 7) / 8);
   const int32_t *w_in = g->w_i32_in.as<int32_t>(), *w_out = g->w_i32_out.as<int32_t>();
   pm_traversal_stats s{};
   E.tag = "bellman_ford_multi";
   for (;;) {
     PM_CUDA(cudaMemsetAsync(E.d_cnt, 0, 3 * sizeof(Counters), E.stream));
-    PM_LAUNCH(k_bf_multi_frontier, E.grid_for(n, 256, 8), 256, 0, E.stream, act, E.g.out.off, n, queue, qdeg,
+    PM_LAUNCH(k_bf_multi_frontier, E.grid_for((n + 3) / 4, 256, 8), 256, 0, E.stream, act, E.g.out.off, n, queue, qdeg,
               E.d_cnt + 1);
     const Counters *h = E.read_counters();
     const int64_t size = (int64_t)h[1].size, edges = (int64_t)h[1].edges, q = (int64_t)h[1].aux;
@@ -394,7 +438,7 @@ void run_bf_multi(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_dist_
     if (dense) {
       if (items > 0)
         PM_LAUNCH(k_bf_multi_pull, pull_grid, 256, 0, E.stream, E.g, w_in, dist, act, nxt, heavy_pieces,
-                  o.order.as<int32_t>(), rh, rl);
+                  o.order.as<int32_t>(), rh, rl, k);
     } else {
       if (q > 0) {
         PM_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, qdeg, qoff, (int)q, E.stream));
