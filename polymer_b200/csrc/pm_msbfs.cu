@@ -21,8 +21,11 @@
 // What bounds it: the first dense level, which has to look at most edges (an
 // 8-byte gather each), and the k x n depths (1 GB for 64 sources at 2^22
 // vertices).  64 sources, symmetrised 2^22-vertex, 128 M-edge R-MAT: 2.80 to
-// 3.23 ms as host-driven rounds of whole-row pulls -> 1.90 ms (the first dense
-// level 0.6 ms, 214 G gathers/s; the depths 0.35 ms).
+// 3.23 ms as host-driven rounds of whole-row pulls -> 1.85 ms (the first dense
+// level 0.6 ms, 214 G gathers/s; the depths 0.2 ms).  Two CTAs per SM: three
+// (40 registers, with spills) take 1.81 ms there, but 0.85 instead of 0.80 ms
+// on a directed 2^21-vertex graph and 0.36 instead of 0.30 on 0.3 M vertices,
+// where the barriers count.
 #include "pm_rounds.cuh"
 #include "pm_sorted.cuh"
 
@@ -207,9 +210,20 @@ __device__ __forceinline__ void msbfs_pull(const GraphView &g, const MsbfsWork &
   }
 }
 
-// Writes the depths of levels [l0, l0 + cnt): cnt <= 16, so a lane's level
-// among them is four bits, kept as four planes of 64 lanes.  first: all k rows
-// are written (-1 where no level has the lane), else only the lanes found.
+// Bit i of a byte at bit 4 i.
+__device__ __forceinline__ unsigned spread_nibbles(unsigned x) {
+  x = (x | x << 12) & 0x000f000fu;
+  x = (x | x << 6) & 0x03030303u;
+  return (x | x << 3) & 0x11111111u;
+}
+
+// Writes the depths of levels [l0, l0 + cnt): cnt < kSlots, so a lane's level
+// among them is four bits, kept as four planes of 64 lanes; fifteen stands for
+// none.  Eight lanes at a time their planes become nibbles (a shift of each
+// 64-bit plane per lane took 350 us of a 1.9 ms call, this about 200).
+// first: all k rows are written (-1 where no level has the lane), else only
+// the lanes found.
+static_assert(kSlots <= 16, "fifteen levels and the mark for none in four bits");
 __device__ __forceinline__ void msbfs_depths(const MsbfsWork &w, int64_t n, int32_t l0, int cnt, bool first) {
   const int64_t gsize = (int64_t)gridDim.x * blockDim.x;
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gsize) {
@@ -224,23 +238,24 @@ __device__ __forceinline__ void msbfs_depths(const MsbfsWork &w, int64_t n, int3
       if (j & 8) p3 |= x;
     }
     if (!first && found == 0) continue;
+    p0 |= ~found;
+    p1 |= ~found;
+    p2 |= ~found;
+    p3 |= ~found;
     int32_t *out = w.depth + v;
-    for (int l = 0; l < w.k; ++l, out += n) {
-      const int32_t d = l0 + (int)(p0 & 1) + 2 * (int)(p1 & 1) + 4 * (int)(p2 & 1) + 8 * (int)(p3 & 1);
-      if (found & 1)
-        *out = d;
-      else if (first)
-        *out = -1;
-      p0 >>= 1;
-      p1 >>= 1;
-      p2 >>= 1;
-      p3 >>= 1;
-      found >>= 1;
+    for (int l = 0; l < w.k; l += 8) {
+      const unsigned q = spread_nibbles((unsigned)(p0 >> l) & 255u) | spread_nibbles((unsigned)(p1 >> l) & 255u) << 1 |
+                         spread_nibbles((unsigned)(p2 >> l) & 255u) << 2 | spread_nibbles((unsigned)(p3 >> l) & 255u) << 3;
+#pragma unroll
+      for (int i = 0; i < 8; ++i, out += n) {
+        const int t = (int)(q >> (4 * i)) & 15;
+        if (l + i < w.k && (first || t != 15)) *out = t == 15 ? -1 : l0 + t;
+      }
     }
   }
 }
 
-__global__ void __launch_bounds__(kRoundThreads, 3) k_msbfs(GraphView g, MsbfsWork w, int64_t threshold) {
+__global__ void __launch_bounds__(kRoundThreads, 2) k_msbfs(GraphView g, MsbfsWork w, int64_t threshold) {
   cg::grid_group grid = cg::this_grid();
   const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, gsize = (int64_t)gridDim.x * blockDim.x;
   const int64_t n = g.n;
