@@ -286,9 +286,11 @@ __global__ void __launch_bounds__(256, kBfCtas) k_bf_multi_pull(GraphView g, con
                                                                 const int32_t *__restrict__ order, int rh, int rl,
                                                                 int k) {
   const int lane = lane_id(), group = lane / kBfSub, t = lane % kBfSub;
-  // threads past the k sources read thread 0's lanes (no further sector) and write nothing
+  // threads past the k sources read the last used thread's lanes, no further
+  // sector, and write nothing (thread 0's, out of order, make the load slower:
+  // 50 sources 4.60 instead of 4.20 ms)
   const bool used = 8 * t < k;
-  const int32_t *col = dist + (used ? 8 * t : 0);
+  const int32_t *col = dist + 8 * min(t, (k - 1) / 8);
   int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (item < heavy_pieces) {
     const int c = (int)(item / (kChunkEdges / kBfPiece));
