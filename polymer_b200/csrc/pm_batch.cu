@@ -31,7 +31,7 @@ using u64 = unsigned long long;
 // issue slots at 22 % of the L2's rate with half a warp per row and a test per
 // lane; a load, two shuffles and eight add-and-minimum instructions per four
 // rows now).  50 sources, 1.5 M vertices, 42 M edges: 9.0 ms with a warp per
-// row in vertex order, 6.65 with half a warp per row by in-degree, 4.33 here
+// row in vertex order, 6.65 with half a warp per row by in-degree, 4.2 here
 // (a dense round 1.25 -> 0.78 ms).
 // ===========================================================================
 constexpr int kLanes = 64;
@@ -43,14 +43,15 @@ constexpr int kBfCtas = 8;
 constexpr int kBfPushUnroll = 2;  // push: out-edges whose target rows are read together per warp
 
 // active -> queue of frontier vertices with out-edges (and their degrees);
-// c->size = |F|, c->edges = outdeg(F), c->aux = queue length.  A block takes
-// 1024 vertices at a time, four side by side per thread, and reserves their
-// queue slots with one atomic (an atomic per warp and 32 vertices took 60 us
-// for a frontier of most of 1.5 M vertices).
+// size = |F|, edges = outdeg(F), aux = queue length, left in *host (pinned) by
+// the last block, which clears c and the ticket for the next round; next is
+// cleared for the round, too.  A block takes 1024 vertices at a time, four side
+// by side per thread, and reserves their queue slots with one atomic (an atomic
+// per warp and 32 vertices took 60 us for a frontier of most of 1.5 M vertices).
 __global__ void __launch_bounds__(256) k_bf_multi_frontier(const u64 *__restrict__ active,
                                                            const int32_t *__restrict__ out_off, int64_t n,
                                                            int32_t *__restrict__ queue, int32_t *__restrict__ qdeg,
-                                                           Counters *c) {
+                                                           u64 *next, Counters *c, u64 *ticket, Counters *host) {
   __shared__ unsigned s_count[8];
   __shared__ unsigned long long s_at, s_size[8], s_edges[8];
   const int lane = lane_id(), wid = threadIdx.x >> 5;
@@ -65,6 +66,7 @@ __global__ void __launch_bounds__(256) k_bf_multi_frontier(const u64 *__restrict
     for (int u = 0; u < U; ++u) {
       const int64_t v = base + u * 256 + threadIdx.x;
       act[u] = v < n && active[v] != 0ull;
+      if (v < n) next[v] = 0ull;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -111,6 +113,14 @@ __global__ void __launch_bounds__(256) k_bf_multi_frontier(const u64 *__restrict
     }
     if (size) atomicAdd(&c->size, size);
     if (edges) atomicAdd(&c->edges, edges);
+    __threadfence();
+    if (atomicAdd(ticket, 1ull) == gridDim.x - 1) {
+      host->size = atomicExch(&c->size, 0ull);
+      host->edges = atomicExch(&c->edges, 0ull);
+      host->aux = atomicExch(&c->aux, 0ull);
+      *ticket = 0ull;
+      __threadfence_system();
+    }
   }
 }
 
@@ -425,18 +435,19 @@ void run_bf_multi(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_dist_
   const int32_t *w_in = g->w_i32_in.as<int32_t>(), *w_out = g->w_i32_out.as<int32_t>();
   pm_traversal_stats s{};
   E.tag = "bellman_ford_multi";
+  PM_CUDA(cudaMemsetAsync(E.d_cnt, 0, 3 * sizeof(Counters), E.stream));
   for (;;) {
-    PM_CUDA(cudaMemsetAsync(E.d_cnt, 0, 3 * sizeof(Counters), E.stream));
+    // a round trip: this launch and a wait (with the counters copied back and
+    // two words cleared by memsets it took about 35 us)
     PM_LAUNCH(k_bf_multi_frontier, E.grid_for((n + 3) / 4, 256, 8), 256, 0, E.stream, act, E.g.out.off, n, queue, qdeg,
-              E.d_cnt + 1);
-    const Counters *h = E.read_counters();
-    const int64_t size = (int64_t)h[1].size, edges = (int64_t)h[1].edges, q = (int64_t)h[1].aux;
+              nxt, E.d_cnt + 1, &E.d_cnt[2].aux, E.h_cnt);
+    PM_CUDA(cudaStreamSynchronize(E.stream));
+    const int64_t size = (int64_t)E.h_cnt->size, edges = (int64_t)E.h_cnt->edges, q = (int64_t)E.h_cnt->aux;
     if (size == 0) break;
     if (s.rounds > n + 1) fail(PM_ERR_INVALID_ARG, "BellmanFord did not converge");
     s.edges_visited += edges;
     const bool dense = size + edges >= threshold;
     E.prof.begin(E.tag, E.stream);
-    PM_CUDA(cudaMemsetAsync(nxt, 0, (size_t)n * 8, E.stream));
     if (dense) {
       if (items > 0)
         PM_LAUNCH(k_bf_multi_pull, pull_grid, 256, 0, E.stream, E.g, w_in, dist, act, nxt, heavy_pieces,
