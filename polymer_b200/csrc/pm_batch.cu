@@ -20,9 +20,8 @@ using u64 = unsigned long long;
 //    each in-edge whose source has active lanes they gather the source's row
 //    and take its minimum with the weight added;
 //  * sparse: the frontier's out-edges are cut into 32-edge chunks (a scan of
-//    the queued out-degrees); for each edge the warp relaxes the active lanes
-//    of the target with atomicMin and ORs the lanes that fell into the
-//    target's next active word.
+//    the queued out-degrees); for each edge eight lanes of the warp relax the
+//    target's with atomicMin and OR those that fell into its next active word.
 // Distances only fall, so reading a row another warp is lowering in the same
 // round is harmless: the lower value is a real path length and the lane that
 // fell is in the next frontier either way.
@@ -31,8 +30,9 @@ using u64 = unsigned long long;
 // issue slots at 22 % of the L2's rate with half a warp per row and a test per
 // lane; a load, two shuffles and eight add-and-minimum instructions per four
 // rows now).  50 sources, 1.5 M vertices, 42 M edges: 9.0 ms with a warp per
-// row in vertex order, 6.65 with half a warp per row by in-degree, 4.2 here
-// (a dense round 1.25 -> 0.78 ms).
+// row in vertex order, 6.65 with half a warp per row by in-degree, 4.0 here
+// (a dense round 1.25 -> 0.72 ms; the pushes, a warp per edge and two in flight
+// before, 0.54 -> about 0.3).
 // ===========================================================================
 constexpr int kLanes = 64;
 // Resident CTAs per SM of the pull: with eight, a row in flight per group of
@@ -40,7 +40,7 @@ constexpr int kLanes = 64;
 // and two rows in flight 4.44, with five and three 4.72, with four and four
 // 4.82.
 constexpr int kBfCtas = 8;
-constexpr int kBfPushUnroll = 2;  // push: out-edges whose target rows are read together per warp
+constexpr int kBfPushCtas = 6;  // of the push (four, two edges in flight per group: 1 % slower)
 
 // active -> queue of frontier vertices with out-edges (and their degrees);
 // size = |F|, edges = outdeg(F), aux = queue length, left in *host (pinned) by
@@ -124,14 +124,43 @@ __global__ void __launch_bounds__(256) k_bf_multi_frontier(const u64 *__restrict
   }
 }
 
-__global__ void __launch_bounds__(256) k_bf_multi_push(const int32_t *__restrict__ out_off,
+// Eight of a row's 64 distances: 32 bytes, one load.
+struct Oct {
+  int32_t x[8];
+};
+__device__ __forceinline__ Oct ld_oct(const int32_t *p) {
+  Oct v;
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]), "=r"(v.x[4]), "=r"(v.x[5]), "=r"(v.x[6]),
+                 "=r"(v.x[7])
+               : "l"(p));
+  return v;
+}
+
+// The same past L1: what other warps' atomics have made of it.
+__device__ __forceinline__ Oct ld_oct_fresh(const int32_t *p) {
+  Oct v;
+  asm volatile("ld.volatile.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3])
+               : "l"(p));
+  asm volatile("ld.volatile.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x[4]), "=r"(v.x[5]), "=r"(v.x[6]), "=r"(v.x[7])
+               : "l"(p + 4));
+  return v;
+}
+
+constexpr int kBfSub = 8;  // lanes per row
+
+// Eight lanes per edge, each group of them eight of the chunk's 32 edges one
+// after another: a warp has four targets' rows in flight.
+__global__ void __launch_bounds__(256, kBfPushCtas) k_bf_multi_push(const int32_t *__restrict__ out_off,
                                                        const int32_t *__restrict__ out_idx,
                                                        const int32_t *__restrict__ w_out,
                                                        const int32_t *__restrict__ queue,
                                                        const int32_t *__restrict__ qoff, int q, int64_t total,
                                                        int32_t *dist, const u64 *__restrict__ active,
                                                        u64 *next_active) {
-  const int lane = lane_id();
+  const int lane = lane_id(), sub = lane % kBfSub;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t chunk = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); chunk * 32 < total;
        chunk += warps) {
@@ -163,66 +192,39 @@ __global__ void __launch_bounds__(256) k_bf_multi_push(const int32_t *__restrict
       d = __ldg(out_idx + e);
       w = __ldg(w_out + e);
     }
-    const int cnt = (int)min((int64_t)32, total - t0);
     int cur = -1;
-    u64 a = 0;
-    int32_t slo = 0, shi = 0;
-    for (int j0 = 0; j0 < cnt; j0 += kBfPushUnroll) {
-      // kBfPushUnroll edges at a time: the targets' rows are read, and their
-      // atomics issued, before any result is waited for.
-      int dj[kBfPushUnroll];
-      int32_t nlo[kBfPushUnroll], nhi[kBfPushUnroll], olo[kBfPushUnroll], ohi[kBfPushUnroll];
+    unsigned on = 0;  // the active lanes among this thread's eight of the source's
+    Oct from;
+    for (int j = 0; j < kBfSub; ++j) {
+      const int sj = __shfl_sync(0xffffffffu, s, j, kBfSub);
+      const int dj = __shfl_sync(0xffffffffu, d, j, kBfSub);
+      const int32_t wj = __shfl_sync(0xffffffffu, w, j, kBfSub);
+      if (sj >= 0 && sj != cur) {
+        cur = sj;
+        on = __ldg(reinterpret_cast<const uint8_t *>(active + sj) + sub);
+        if (on) from = ld_oct(dist + (int64_t)sj * kLanes + 8 * sub);
+      }
+      if (sj < 0 || !on) continue;
+      // A lane below the distance read here lowers it with an atomic whose
+      // result is unused and is marked active: it fell, or another push
+      // lowered it further meanwhile (an extra relaxation next round, the same
+      // distances).
+      int32_t *to = dist + (int64_t)dj * kLanes + 8 * sub;
+      const Oct old = ld_oct_fresh(to);
+      unsigned fell = 0;
 #pragma unroll
-      for (int u = 0; u < kBfPushUnroll; ++u) {
-        const int j = min(j0 + u, cnt - 1);
-        const bool take = j0 + u < cnt;
-        const int sj = __shfl_sync(0xffffffffu, s, j);
-        dj[u] = __shfl_sync(0xffffffffu, d, j);
-        const int32_t wj = __shfl_sync(0xffffffffu, w, j);
-        if (sj != cur) {
-          cur = sj;
-          a = __ldg(active + sj);
-          slo = dist[(int64_t)sj * kLanes + lane];
-          shi = dist[(int64_t)sj * kLanes + 32 + lane];
+      for (int i = 0; i < 8; ++i) {
+        const int32_t nv = on >> i & 1u ? from.x[i] + wj : kDevBFInf;
+        if (nv < kDevBFInf && nv < old.x[i]) {
+          atomicMin(to + i, nv);
+          fell |= 1u << i;
         }
-        nlo[u] = take && ((a >> lane) & 1ull) ? slo + wj : kDevBFInf;
-        nhi[u] = take && ((a >> (32 + lane)) & 1ull) ? shi + wj : kDevBFInf;
-        olo[u] = nlo[u] < kDevBFInf ? *(volatile int32_t *)(dist + (int64_t)dj[u] * kLanes + lane) : 0;
-        ohi[u] = nhi[u] < kDevBFInf ? *(volatile int32_t *)(dist + (int64_t)dj[u] * kLanes + 32 + lane) : 0;
       }
-      // A lane below the distance read above lowers it with an atomic
-      // whose result is unused and is marked active: it fell, or another
-      // push lowered it further meanwhile (an extra relaxation next round,
-      // the same distances).
-#pragma unroll
-      for (int u = 0; u < kBfPushUnroll; ++u) {
-        if (nlo[u] < olo[u]) atomicMin(dist + (int64_t)dj[u] * kLanes + lane, nlo[u]);
-        if (nhi[u] < ohi[u]) atomicMin(dist + (int64_t)dj[u] * kLanes + 32 + lane, nhi[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < kBfPushUnroll; ++u) {
-        const u64 mask = (u64)__ballot_sync(0xffffffffu, nlo[u] < olo[u]) |
-                         ((u64)__ballot_sync(0xffffffffu, nhi[u] < ohi[u]) << 32);
-        if (lane == 0 && mask) atomicOr(next_active + dj[u], mask);
-      }
+      if (fell) atomicOr(reinterpret_cast<unsigned *>(next_active + dj) + sub / 4, fell << 8 * (sub % 4));
     }
   }
 }
 
-// Eight of a row's 64 distances: 32 bytes, one load.
-struct Oct {
-  int32_t x[8];
-};
-__device__ __forceinline__ Oct ld_oct(const int32_t *p) {
-  Oct v;
-  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v.x[0]), "=r"(v.x[1]), "=r"(v.x[2]), "=r"(v.x[3]), "=r"(v.x[4]), "=r"(v.x[5]), "=r"(v.x[6]),
-                 "=r"(v.x[7])
-               : "l"(p));
-  return v;
-}
-
-constexpr int kBfSub = 8;  // lanes per row
 constexpr int kBfSmallWeight = 1 << 30;
 
 // The least dist[s] + w over this group's in-edges whose sources have active
