@@ -53,8 +53,8 @@ def parse():
     p.add_argument("--no-tune", action="store_true",
                    help="keep the default tunables instead of running the autotuner at setup")
     p.add_argument("--no-cuda-graphs", action="store_true",
-                   help="launch every kernel directly (the same work): for profilers that cannot see "
-                        "kernels inside CUDA graphs with conditional nodes (the device-driven BFS rounds)")
+                   help="launch every kernel directly (the same work; BFS rounds driven by the host): for "
+                        "profilers that cannot see kernels inside CUDA graphs")
     return p.parse_args()
 
 
@@ -214,7 +214,8 @@ class Suite:
         bytes]} into per.  Bytes per call: BFS 4 E_r + 12 n (E_r: out-degrees of
         the reached vertices); CC sum over rounds of 8 E_F + 12 n and
         BellmanFord of 12 E_F + 12 n (E_F: the round's frontier out-degrees);
-        PageRank 8 m + 32 n, SpMV 12 m + 12 n, BP 4 m + 40 n per iteration."""
+        PageRank 8 m + 32 n, SpMV 12 m + 12 n per iteration; BP 4 m once (the counts of
+        messages) + 40 n per iteration."""
         pm, A, B = self.pm, self.A, self.B
         total_ms, total_edges = 0.0, 0
         nA, nB, mB = A.n, B.n, B.m
@@ -246,7 +247,7 @@ class Suite:
         rec("spmv", B.timer_end(), mB * 10, (12 * mB + 12 * nB) * 10)
         B.timer_begin()
         pm.BeliefPropagation(B, self.prior, 10)
-        rec("bp", B.timer_end(), mB * 10, (4 * mB + 40 * nB) * 10)
+        rec("bp", B.timer_end(), mB * 10, 4 * mB + 40 * nB * 10)
         return total_ms, total_edges
 
 
@@ -672,7 +673,7 @@ def adjoint_block(pm, torch, dev, reps=3):
 
 def ncu_traffic():
     """DRAM bytes per PageRank pass from the committed ncu summary, if any."""
-    path = os.path.join(ROOT, "profiles", "pagerank_pull_rmat24.md")
+    path = os.path.join(ROOT, "profiles", "sorted_pull_rmat24.md")
     try:
         for ln in open(path):
             if ln.strip().startswith("traffic_bytes_per_pass:"):
@@ -913,16 +914,16 @@ def main():
         "config": suite_config(args.scale_a, args.scale_b, len(suite.sources), suite.A.n, suite.A.m, nB, mB,
                                world),
         "launch": "direct launches (--no-cuda-graphs)" if args.no_cuda_graphs else
-                  "CUDA graphs: captured PageRank/SpMV/BP loops, device-driven BFS rounds",
+                  "CUDA graphs: captured PageRank/SpMV loops; traversals and BP one cooperative launch each",
         "per_algo": per_algo,
         "roofline": {
-            "kernel": "PageRank pull-reduce pass (k_heavy_reduce + k_pull_reduce<PR_F<float>>)",
+            "kernel": "PageRank pass over the degree-sorted copy (k_sorted_pull<PRS_F<float>>)",
             "bound": "hbm", "achieved": round(achieved, 1) if achieved else None,
             "peak": hbm, "peak_kind": peak_kind, "unit": "GB/s",
             "frac": round(achieved / hbm, 4) if achieved else None,
             "traffic": ncu_traffic(),
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the pass, from the "
-                              "committed summary profiles/pagerank_pull_rmat24.md (not measured in this run)",
+                              "committed summary profiles/sorted_pull_rmat24.md (not measured in this run)",
             "algorithmic_bytes_per_pass": pass_bytes,
             "algorithmic_bytes_rule": "8 m + 16 n: CSC id + gathered contribution per edge; offset, "
                                       "out-degree, rank write, contribution write per vertex",

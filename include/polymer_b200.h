@@ -420,7 +420,14 @@ PM_API pm_status pm_profile_read(pm_graph *g, const char *tag, double *total_ms,
  * which fixes its load-balance cut-offs at compile time and passes each
  * application's direction-switch threshold in code (BFS 0, numa-BFS.C:268;
  * CC m/8, numa-Components.C:226; BellmanFord m/20, numa-BellmanFord.C:182).
- * Results never depend on them; only speed does. */
+ * Results never depend on them; only speed does.
+ * On a whole-graph handle PageRank, SpMV, BP, the weighted fixed points and
+ * PPR run over a copy sorted by degree (or, BP, over counts), which takes none
+ * of HEAVY_DEG, PULL_CTAS_PER_SM, HEAVY_MODE, HUB_CACHE and PULL_STAGE; these
+ * remain for the vertex-order pulls: partitions, handles without room for the
+ * copy, PageRankDelta, a damping outside [0, 1], and the pull rounds of
+ * Components and BellmanFord.  HEAVY_DEG also cuts multi-source BellmanFord's
+ * rows. */
 #define PM_TUNE_HEAVY_DEG 0        /* rows with more edges are split in 4096-edge chunks
                                       (default 1024, range [64, 2^30]) */
 #define PM_TUNE_CTA_EXPAND 1       /* sparse push: CTA-wide expansion from this
@@ -434,18 +441,19 @@ PM_API pm_status pm_profile_read(pm_graph *g, const char *tag, double *total_ms,
 #define PM_TUNE_CC_DIV 5           /* ... Components (default 8) */
 #define PM_TUNE_BF_DIV 6           /* ... BellmanFord (default 20) */
 #define PM_TUNE_CUDA_GRAPHS 7      /* 1 (default): the fixed-iteration loops of PageRank,
-                                      SpMV, BP and PPR run as CUDA graphs, captured the
+                                      SpMV and PPR run as CUDA graphs, captured the
                                       second time a handle runs the same loop (same
                                       sizes, buffers and scalars) and replayed from
-                                      then on, and BFS runs its rounds inside one CUDA
-                                      graph whose WHILE node chooses each round's
-                                      direction on the GPU; 0: plain launches */
+                                      then on, and BFS runs all its rounds in one
+                                      cooperative launch that chooses each round's
+                                      direction on the GPU; 0: plain launches, BFS
+                                      driven by the host */
 #define PM_TUNE_HEAVY_MODE 8       /* how the chunks of heavy rows are summed: 0 (default)
                                       a launch before the pull; 1 inside the pull launch
                                       (warps take them first, a row's lane waits for its
                                       chunks, bounded); 2 a launch beside the pull on a
                                       second stream, the heavy rows committed after both */
-#define PM_TUNE_HUB_CACHE 9        /* FP32 PageRank: the contributions of up to this many
+#define PM_TUNE_HUB_CACHE 9        /* FP32 PageRank in vertex order: the contributions of up to this many
                                       highest out-degree sources are kept in every SM's
                                       shared memory during a pass (0 = off, the default; at
                                       most 16384; results are unchanged; slower than the
