@@ -7,6 +7,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "pm_edges.cuh"
 #include "polymer_b200.h"
 
 // C++ symbols the engine templates call from code compiled outside the

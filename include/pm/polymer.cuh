@@ -457,9 +457,9 @@ __global__ void __launch_bounds__(256) k_dense_pull(GraphView g, const uint32_t 
     int v = (int)t;
     bool act = false, deferred = false;
     if (v < g.n && f.cond(v)) {
-      int o0 = __ldg(g.in.off + v), o1 = __ldg(g.in.off + v + 1);
-      int lim = min(o1, o0 + kPullScan);
-      int e = o0;
+      const EdgePos o0 = __ldg(g.in.off + v), o1 = __ldg(g.in.off + v + 1);
+      const EdgePos lim = edge_end(o0, kPullScan, o1);
+      EdgePos e = o0;
       for (; e < lim; ++e) {
         int s = checked_id(g, __ldg(g.in.idx + e));
         if (test_bit(cur, s) && update_atomic(f, s, v, load_w(w, e))) act = true;
@@ -502,10 +502,10 @@ __global__ void __launch_bounds__(256) k_dense_pull_defer(GraphView g,
   const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t k = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < nd; k += nwarps) {
     int v = defer[k];
-    int o0 = __ldg(g.in.off + v) + kPullScan, o1 = __ldg(g.in.off + v + 1);
+    const EdgePos o0 = (EdgePos)__ldg(g.in.off + v) + kPullScan, o1 = __ldg(g.in.off + v + 1);
     bool act = false, open = true;
-    for (int base = o0; base < o1 && open; base += 32) {
-      int e = base + lane;
+    for (EdgePos base = o0; base < o1 && open; base += 32) {
+      const EdgePos e = base + lane;
       int s = e < o1 ? checked_id(g, __ldg(g.in.idx + e)) : 0;
       unsigned bal = __ballot_sync(0xffffffffu, e < o1 && test_bit(cur, s));
       while (bal && open) {
@@ -1005,7 +1005,7 @@ __global__ void __launch_bounds__(HUBS ? kHubBlock : kPullBlock, HUBS ? 2 : PM_P
     if constexpr (MODE == 2) deferred = live && heavy;
     if (live && heavy && !deferred) {
       const int first = __ldg(g.in.hfirst + r);
-      const int nch = (deg + kChunkEdges - 1) / kChunkEdges;
+      const int nch = edge_pieces(deg, kChunkEdges);
       if constexpr (MODE == 1) {
         wait_at_least(hdone + first, nch, kHeavyWaitSpins, &cnt->err);
         for (int k = 0; k < nch; ++k) acc = f.combine(acc, __ldcg(partials + first + k));
@@ -1052,7 +1052,7 @@ __global__ void __launch_bounds__(256) k_heavy_commit(GraphView g, F f, const ty
     const int first = __ldg(g.in.hfirst + r);
     if (c != first || !f.cond(r)) continue;
     const int deg = __ldg(g.in.off + r + 1) - __ldg(g.in.off + r);
-    const int nch = (deg + kChunkEdges - 1) / kChunkEdges;
+    const int nch = edge_pieces(deg, kChunkEdges);
     Acc acc = f.identity();
     for (int k = 0; k < nch; ++k) acc = f.combine(acc, partials[first + k]);
     if (f.commit(r, acc, my_aux)) {

@@ -53,7 +53,7 @@ __global__ void k_async_init(unsigned long long *queue, int64_t cap, int32_t *pa
 // The source's items (one per chunk of its out-edges), before the traversal.
 __global__ void k_async_seed(GraphView g, unsigned long long *queue, int src, AsyncCtl *ctl) {
   const int deg = g.out.off[src + 1] - g.out.off[src];
-  const int nch = (deg + kAsyncChunk - 1) / kAsyncChunk;
+  const int nch = edge_pieces(deg, kAsyncChunk);
   for (int c = 0; c < nch; ++c) queue[c] = item_of(src, c);
   ctl->head = 0;
   ctl->tail = (unsigned long long)nch;
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(256) k_bfs_async(GraphView g, int32_t *parents
       int dnch = 0;
       if (claimed) {
         const int ddeg = __ldg(g.out.off + d + 1) - __ldg(g.out.off + d);
-        dnch = ddeg > 0 ? (ddeg + kAsyncChunk - 1) / kAsyncChunk : 0;
+        dnch = edge_pieces(ddeg, kAsyncChunk);
         my_reached++;
       }
       warp_enqueue(dnch > 0, item_of(d, 0), queue, cap, ctl);

@@ -238,8 +238,8 @@ constexpr int kBfSmallWeight = 1 << 30;
 // the places without an edge.  All lanes of the warp call it; the groups may
 // have different rows and lengths.  col: dist at this thread's lanes.
 __device__ __forceinline__ Oct bf_multi_relax(const int32_t *__restrict__ in_idx, const int32_t *__restrict__ w_in,
-                                              const int32_t *col, const u64 *__restrict__ active, int self, int e,
-                                              int e1, int step) {
+                                              const int32_t *col, const u64 *__restrict__ active, int self, EdgePos e,
+                                              EdgePos e1, int step) {
   const int t = lane_id() & 7, shift = lane_id() & 24;
   Oct m;
 #pragma unroll
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(256, kBfCtas) k_bf_multi_pull(GraphView g, con
     const int64_t first = (int64_t)__ldg(g.in.off + r) + (int64_t)(c - __ldg(g.in.hfirst + r)) * kChunkEdges +
                           (int64_t)piece * kBfPiece;
     if (first >= row_end) return;
-    const int e0 = (int)first, e1 = min(row_end - e0, kBfPiece) + e0;
+    const EdgePos e0 = (EdgePos)first, e1 = edge_end(e0, kBfPiece, row_end);
     const Oct m = bf_multi_join(bf_multi_relax(g.in.idx, w_in, col, active, r, e0 + kBfSub * group, e1, 32));
     if (group != 0 || !used) return;
     unsigned fell = 0;
@@ -326,13 +326,14 @@ __global__ void __launch_bounds__(256, kBfCtas) k_bf_multi_pull(GraphView g, con
   item -= heavy_pieces;
   const bool whole = item < rh;  // the same for the whole warp
   const int64_t r = whole ? item : rh + (32 / kBfSub) * (item - rh) + group;
-  int v = 0, e0 = 0, e1 = 0;
+  int v = 0;
+  EdgePos e0 = 0, e1 = 0;
   bool mine = r < rl;
   if (mine) {
     v = __ldg(order + r);
     e0 = __ldg(g.in.off + v);
     e1 = __ldg(g.in.off + v + 1);
-    mine = e1 - e0 <= g.heavy_deg;
+    mine = e1 - e0 <= (EdgePos)g.heavy_deg;
     if (!mine) e1 = e0;
   }
   if (!__any_sync(0xffffffffu, mine)) return;

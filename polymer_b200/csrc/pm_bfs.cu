@@ -39,7 +39,8 @@ __device__ __forceinline__ void bfs_pull(const GraphView &g, const BfsWork &w, c
   const int64_t ntot = ((int64_t)g.n + 31) & ~31ll, gsize = (int64_t)gridDim.x * blockDim.x;
   auto in_cur = [&](int s) { return s >= 0 && ((cur[s >> 5] >> (s & 31)) & 1u); };
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < ntot; t += kStep * gsize) {
-    int parent[kStep], e[kStep], e1[kStep];
+    int parent[kStep];
+    EdgePos e[kStep], e1[kStep];
 #pragma unroll
     for (int u = 0; u < kStep; ++u) parent[u] = t + u * gsize < g.n ? w.parents[t + u * gsize] : 0;
 #pragma unroll
@@ -63,14 +64,14 @@ __device__ __forceinline__ void bfs_pull(const GraphView &g, const BfsWork &w, c
       for (int u = 0; u < kStep; ++u) {
         const bool ha = in_cur(a[u]), hb = in_cur(b[u]);
         parent[u] = ha ? a[u] : hb ? b[u] : -1;
-        e[u] = min(e[u] + 2, e1[u]);
+        e[u] = edge_end(e[u], 2, e1[u]);
       }
     }
 #pragma unroll
     for (int u = 0; u < kStep; ++u) {
       if (t - lane + u * gsize >= ntot) break;  // the same for the whole warp
       const int v = (int)(t + u * gsize);
-      const int lim = min(e1[u], e[u] + kPullScan);
+      const EdgePos lim = edge_end(e[u], kPullScan, e1[u]);
       while (e[u] < lim && parent[u] < 0) {
         int s[kStep];
         bool hit[kStep];
@@ -81,21 +82,21 @@ __device__ __forceinline__ void bfs_pull(const GraphView &g, const BfsWork &w, c
 #pragma unroll
         for (int k = kStep - 1; k >= 0; --k)
           if (hit[k]) parent[u] = s[k];
-        e[u] = min(e[u] + kStep, lim);
+        e[u] = edge_end(e[u], kStep, lim);
       }
       // rows still open: the warp scans each together
       unsigned open = __ballot_sync(0xffffffffu, parent[u] < 0 && e[u] < e1[u]);
       while (open) {
         const int l = __ffs(open) - 1;
         open &= open - 1;
-        const int o1 = __shfl_sync(0xffffffffu, e1[u], l);
+        const EdgePos o1 = __shfl_sync(0xffffffffu, e1[u], l);
         int found = -1;
-        for (int o = __shfl_sync(0xffffffffu, e[u], l); o < o1 && found < 0; o += 32 * kStep) {
+        for (EdgePos o = __shfl_sync(0xffffffffu, e[u], l); o < o1 && found < 0; o += 32 * kStep) {
           int s[kStep];
           bool hit[kStep];
 #pragma unroll
           for (int k = 0; k < kStep; ++k) {
-            const int x = o + 32 * k + lane;
+            const EdgePos x = o + 32 * k + lane;
             s[k] = x < o1 ? checked_id(g, __ldg(g.in.idx + x)) : -1;
           }
 #pragma unroll
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_bfs(GraphView g, BfsWork w
       }
       round_push(
           g, q, f.rows, f.pieces, [](int s) { return s; },
-          [&](const int (&s)[kStep], const int (&)[kStep], const int (&d)[kStep], const bool (&ok)[kStep]) {
+          [&](const int (&s)[kStep], const EdgePos (&)[kStep], const int (&d)[kStep], const bool (&ok)[kStep]) {
             bool act[kStep];
             int deg[kStep];
 #pragma unroll

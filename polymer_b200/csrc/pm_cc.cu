@@ -192,9 +192,9 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_uf(GraphView g, int32_t *p
         const int l = __ffs(todo) - 1;
         todo &= todo - 1;
         const int32_t v = (int32_t)(base + u * gsize + l);
-        const int32_t e1 = __shfl_sync(0xffffffffu, o1[u], l);
-        const int32_t first = __shfl_sync(0xffffffffu, o0[u], l);
-        for (int32_t e = first + lane; e < e1; e += 32) {
+        const EdgePos e1 = __shfl_sync(0xffffffffu, o1[u], l);
+        const EdgePos first = __shfl_sync(0xffffffffu, o0[u], l);
+        for (EdgePos e = first + lane; e < e1; e += 32) {
           uf_link(parent, v, checked_id(g, __ldg(g.out.idx + e)));
           mine += e >= first + 2;  // the first two were counted above
         }

@@ -124,7 +124,7 @@ __global__ void k_heavy_counts(const int32_t *off, int64_t n, int32_t heavy_deg,
   int32_t md = 0;
   GRID_STRIDE(v, n) {
     int32_t d = off[v + 1] - off[v];
-    nch[v] = d > heavy_deg ? (d + kChunkEdges - 1) / kChunkEdges : 0;
+    nch[v] = d > heavy_deg ? edge_pieces(d, kChunkEdges) : 0;
     md = max(md, d);
   }
   atomicMax(maxdeg, md);

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_min_rounds(GraphView g, co
       }
       grid.sync();
       round_push(g, q, f.rows, f.pieces, value_of,
-                 [&](const int (&x)[kStep], const int (&e)[kStep], const int (&d)[kStep], const bool (&ok)[kStep]) {
+                 [&](const int (&x)[kStep], const EdgePos (&e)[kStep], const int (&d)[kStep], const bool (&ok)[kStep]) {
                    int32_t nv[kStep], seen[kStep];
 #pragma unroll
                    for (int u = 0; u < kStep; ++u) nv[u] = x[u] + (W && ok[u] ? __ldg(weight + e[u]) : 0);
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_min_rounds(GraphView g, co
     } else {
       unsigned long long size = 0, edges = 0;
       round_push(g, q, f.rows, f.pieces, value_of,
-                 [&](const int (&x)[kStep], const int (&e)[kStep], const int (&d)[kStep], const bool (&ok)[kStep]) {
+                 [&](const int (&x)[kStep], const EdgePos (&e)[kStep], const int (&d)[kStep], const bool (&ok)[kStep]) {
                    bool act[kStep];
                    int deg[kStep];
                    int32_t nv[kStep];

@@ -66,7 +66,7 @@ __device__ __forceinline__ u64 lanes_or(u64 x) {
 // WIDTH lanes' common row; all lanes of the warp call it (rows may differ by
 // group), lanes whose row is done wait.
 template <int WIDTH>
-__device__ __forceinline__ u64 msbfs_scan(const GraphView &g, const u64 *front, u64 need, int e, int e1) {
+__device__ __forceinline__ u64 msbfs_scan(const GraphView &g, const u64 *front, u64 need, EdgePos e, EdgePos e1) {
   u64 got = 0;
   bool open = need != 0 && e1 > 0;
   while (__any_sync(0xffffffffu, open)) {
@@ -118,9 +118,9 @@ __device__ __forceinline__ void msbfs_pull(const GraphView &g, const MsbfsWork &
     }
     const u64 need = full & ~vis;
     if (need == 0) continue;
-    const int e1 = min(__ldg(g.in.off + pc.x + 1), pc.y + kOrderPiece);
+    const EdgePos e1 = edge_end((EdgePos)pc.y, kOrderPiece, (EdgePos)__ldg(g.in.off + pc.x + 1));
     u64 x = 0;
-    for (int e = pc.y + threadIdx.x; e < e1; e += kStep * kRoundThreads) {
+    for (EdgePos e = (EdgePos)pc.y + threadIdx.x; e < e1; e += kStep * kRoundThreads) {
       int s[kStep];
 #pragma unroll
       for (int u = 0; u < kStep; ++u)
@@ -142,7 +142,8 @@ __device__ __forceinline__ void msbfs_pull(const GraphView &g, const MsbfsWork &
     const bool whole = t < n1;  // the same for the whole warp
     const int r = whole ? w.rc + (int)t : w.rh + (int)((t - n1) * (32 / kSubLanes)) + lane / kSubLanes;
     const int sub = whole ? lane : lane % kSubLanes;
-    int v = 0, o = 0, o1 = 0;
+    int v = 0;
+    EdgePos o = 0, o1 = 0;
     u64 need = 0;
     if (r < (whole ? w.rh : w.rm)) {
       v = w.order[r];
@@ -170,7 +171,7 @@ __device__ __forceinline__ void msbfs_pull(const GraphView &g, const MsbfsWork &
   // they took three quarters of a level)
   for (int64_t v0 = gtid; v0 < g.n; v0 += kStep * gsize) {
     u64 need[kStep], got[kStep];
-    int o[kStep], o1[kStep];
+    EdgePos o[kStep], o1[kStep];
 #pragma unroll
     for (int u = 0; u < kStep; ++u) {
       const int64_t v = v0 + u * gsize;
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_msbfs(GraphView g, MsbfsWo
       unsigned *nt = w.ntouched + level % 3;
       round_push(
           g, q, f.rows, f.pieces, [&](int s) { return s; },
-          [&](const int (&s)[kStep], const int (&)[kStep], const int (&d)[kStep], const bool (&ok)[kStep]) {
+          [&](const int (&s)[kStep], const EdgePos (&)[kStep], const int (&d)[kStep], const bool (&ok)[kStep]) {
             bool act[kStep];
             int deg[kStep];
             u64 x[kStep];

@@ -282,9 +282,9 @@ __global__ void __cluster_dims__(kPartCluster, 1, 1) __launch_bounds__(kPartThre
     float *A = pc, *B = pn, *cc = c0, *cn = c1;
     for (int it = 0; it < iters; ++it) {
       for (int64_t v = first; v < v1; v += stride) {
-        const int e0 = __ldg(g.in.off + v), e1 = __ldg(g.in.off + v + 1);
+        const EdgePos e0 = __ldg(g.in.off + v), e1 = __ldg(g.in.off + v + 1);
         float acc = -0.0f;
-        int e = e0;
+        EdgePos e = e0;
         for (; e + 3 < e1; e += 4) {
           const int s0 = __ldg(g.in.idx + e), s1 = __ldg(g.in.idx + e + 1);
           const int s2 = __ldg(g.in.idx + e + 2), s3 = __ldg(g.in.idx + e + 3);

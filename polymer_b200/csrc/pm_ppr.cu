@@ -65,7 +65,7 @@ __device__ __forceinline__ Quad xor_add4(Quad a) {  // over the groups of COLS /
 // and lengths.
 constexpr int kPprStep = 4;
 template <int COLS>
-__device__ __forceinline__ Quad ppr_sum(const int32_t *__restrict__ idx, int e, int e1, int step,
+__device__ __forceinline__ Quad ppr_sum(const int32_t *__restrict__ idx, EdgePos e, EdgePos e1, int step,
                                         const float *__restrict__ c, int zero) {
   constexpr int L = COLS / 4, U = kPprStep;      // lanes per row; gathers per step
   constexpr int B = L > U ? L : U, I = B / L;    // edges and id loads per batch
@@ -76,7 +76,7 @@ __device__ __forceinline__ Quad ppr_sum(const int32_t *__restrict__ idx, int e, 
     int id[I];
 #pragma unroll
     for (int i = 0; i < I; ++i) {
-      const int x = e + (i * L + sub) * step;
+      const EdgePos x = e + (i * L + sub) * step;
       id[i] = x < e1 ? __ldcs(idx + x) : zero;
     }
 #pragma unroll
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(256) k_ppr_heavy(GraphView g, const float *__r
   const int k = ch - __ldg(g.in.hfirst + r);
   const int row_end = __ldg(g.in.off + r + 1);
   const int e0 = __ldg(g.in.off + r) + k * kChunkEdges, e1 = min(row_end - e0, kChunkEdges) + e0;
-  const Quad sum = xor_add4<COLS>(ppr_sum<COLS>(g.in.idx, e0 + (int)threadIdx.x / L, e1, 256 / L, c, g.n));
+  const Quad sum = xor_add4<COLS>(ppr_sum<COLS>(g.in.idx, (EdgePos)e0 + threadIdx.x / L, e1, 256 / L, c, g.n));
   if (lane < L) s_part[wid][lane] = sum;
   __syncthreads();
   if (wid == 0 && lane < L) {
@@ -173,11 +173,11 @@ __global__ void __launch_bounds__(256, COLS == 32 ? 8 : 6) k_ppr_pull(GraphView 
     const int o = __ldg(g.in.off + v), o1 = __ldg(g.in.off + v + 1);
     Quad acc{0, 0};
     if (o1 - o > g.heavy_deg) {
-      const int first = __ldg(g.in.hfirst + v), nch = (o1 - o + kChunkEdges - 1) / kChunkEdges;
+      const int first = __ldg(g.in.hfirst + v), nch = edge_pieces(o1 - o, kChunkEdges);
       for (int q = 0; q < nch; ++q)
         add4(acc, ldg4(partials + ((int64_t)(first + q) * L + lane % L) * 4));
     } else {
-      acc = xor_add4<COLS>(ppr_sum<COLS>(g.in.idx, o + group, o1, 32 / L, c_cur, g.n));
+      acc = xor_add4<COLS>(ppr_sum<COLS>(g.in.idx, (EdgePos)o + group, o1, 32 / L, c_cur, g.n));
     }
     if (lane < L) ppr_commit<COLS>(g, v, unpack4(acc), seed, damping, c_next, y_out, k_out);
   } else {

@@ -38,7 +38,7 @@ inline size_t round_pieces(int64_t m) { return (size_t)(m / kShortRow + m / kPus
 
 constexpr int kStep = 4;  // edges or vertices a lane has in flight
 
-__device__ __forceinline__ int round_pieces_of(int deg) { return (deg + kPushChunk - 1) / kPushChunk; }
+__device__ __forceinline__ int round_pieces_of(int deg) { return edge_pieces(deg, kPushChunk); }
 
 // Writes the pieces of the lanes' long rows (n pieces of v from slot at on):
 // a lane writes a few itself, a hub's are written by the whole warp.
@@ -208,17 +208,18 @@ __device__ __forceinline__ void round_push(const GraphView &g, const RoundQueue 
   const unsigned parts = pieces <= warps / 8 ? 8 : pieces <= warps / 2 ? 2 : 1, part_len = kPushChunk / parts;
   for (unsigned i = warp; i < pieces * parts; i += warps) {
     const int2 p = q.pieces[i / parts];
-    const int o = __ldg(g.out.off + p.x), row_end = __ldg(g.out.off + p.x + 1);
+    const EdgeSpan share =
+        edge_share(__ldg(g.out.off + p.x), __ldg(g.out.off + p.x + 1), (EdgePos)p.y, i % parts, part_len);
     const int x = src(p.x);
-    const int e0 = o + p.y + (int)(i % parts * part_len), e1 = min(row_end, e0 + (int)part_len);
-    for (int b = e0; b < e1; b += 32 * kStep) {
-      int xs[kStep], e[kStep], d[kStep];
+    for (EdgePos b = share.begin; b < share.end; b += 32 * kStep) {
+      int xs[kStep], d[kStep];
+      EdgePos e[kStep];
       bool ok[kStep];
 #pragma unroll
       for (int u = 0; u < kStep; ++u) {
         xs[u] = x;
         e[u] = b + 32 * u + lane;
-        ok[u] = e[u] < e1;
+        ok[u] = e[u] < share.end;
         d[u] = ok[u] ? checked_id(g, __ldg(g.out.idx + e[u])) : 0;
       }
       relax(xs, e, d, ok);
@@ -236,7 +237,8 @@ __device__ __forceinline__ void round_push(const GraphView &g, const RoundQueue 
     int total;
     const int pos = warp_excl_scan(deg, &total);
     for (int b = 0; b < total; b += 32 * kStep) {
-      int xs[kStep], e[kStep], d[kStep];
+      int xs[kStep], d[kStep];
+      EdgePos e[kStep];
       bool ok[kStep];
 #pragma unroll
       for (int u = 0; u < kStep; ++u) {
@@ -248,7 +250,7 @@ __device__ __forceinline__ void round_push(const GraphView &g, const RoundQueue 
           for (int step = 16; step > 0; step >>= 1)
             if (__shfl_sync(0xffffffffu, pos, j + step) <= k) j += step;
           xs[u] = __shfl_sync(0xffffffffu, x, j);
-          e[u] = __shfl_sync(0xffffffffu, o, j) + (k - __shfl_sync(0xffffffffu, pos, j));
+          e[u] = (EdgePos)__shfl_sync(0xffffffffu, o, j) + (EdgePos)(k - __shfl_sync(0xffffffffu, pos, j));
         }
         d[u] = ok[u] ? checked_id(g, __ldg(g.out.idx + e[u])) : 0;
       }

@@ -47,15 +47,16 @@ __global__ void k_sort_tables(const int32_t *order, const int32_t *src_off, cons
       bdeg[p - rm] = (uint8_t)d;
       if (((p - rm) & 31) == 0) len[rm + (p - rm) / 32] = 32 * d;
     }
-    if (p < rc) pieces[p] = (d + piece - 1) / piece;
+    if (p < rc) pieces[p] = edge_pieces(d, piece);
   }
 }
 
 __global__ void k_sort_pieces(const int32_t *pfirst, const int32_t *off, int32_t rc, int32_t piece, int4 *pieces) {
   GRID_STRIDE(r, rc) {
-    const int32_t k0 = pfirst[r], k1 = pfirst[r + 1], end = off[r + 1];
-    for (int32_t k = k0, e = off[r]; k < k1; ++k, e += piece)
-      pieces[k] = make_int4(e, min(end - e, piece) + e, (int32_t)r, k1 - k0 > 1 ? k0 : -1);
+    const int32_t k0 = pfirst[r], k1 = pfirst[r + 1];
+    EdgePos e = off[r];
+    for (int32_t k = k0; k < k1; ++k, e += piece)
+      pieces[k] = make_int4((int)e, (int)edge_end(e, piece, off[r + 1]), (int32_t)r, k1 - k0 > 1 ? k0 : -1);
   }
 }
 
@@ -137,11 +138,12 @@ __global__ void k_order_pieces(const int32_t *order, const int32_t *src_off, con
                                int2 *pieces) {
   GRID_STRIDE(r, rc) {
     const int32_t v = order[r];
-    for (int32_t k = first[r], e = src_off[v]; k < first[r + 1]; ++k, e += kOrderPiece) pieces[k] = make_int2(v, e);
+    EdgePos e = src_off[v];
+    for (int32_t k = first[r]; k < first[r + 1]; ++k, e += kOrderPiece) pieces[k] = make_int2(v, (int)e);
   }
 }
 __global__ void k_order_counts(const int32_t *deg, int32_t rc, int32_t *count) {
-  GRID_STRIDE(r, rc + 1) count[r] = r < rc ? (deg[r] + kOrderPiece - 1) / kOrderPiece : 0;
+  GRID_STRIDE(r, rc + 1) count[r] = r < rc ? edge_pieces(deg[r], kOrderPiece) : 0;
 }
 
 const RowOrder &ensure_row_order(pm_graph *g, bool csr) {

@@ -97,7 +97,7 @@ __global__ void k_static_validate(const int32_t *__restrict__ off, const int32_t
       bad |= kBadOffsets;
       continue;
     }
-    for (int32_t e = e0 + lane; e < e1; e += 32) {
+    for (EdgePos e = (EdgePos)e0 + lane; e < (EdgePos)e1; e += 32) {
       const int32_t d = idx[e];
       if (d < 0 || (int64_t)d >= n) bad |= kBadId;
       else if (d == (int32_t)s) bad |= kSelfLoop;
@@ -138,7 +138,7 @@ __global__ void k_static_push(const int32_t *__restrict__ off, const int32_t *__
     const int32_t e0 = off[s], e1 = off[s + 1];
     if (e1 == e0) continue;
     const float c = p_curr[s] / (float)(e1 - e0);
-    for (int32_t e = e0 + lane; e < e1; e += 32) {
+    for (EdgePos e = (EdgePos)e0 + lane; e < (EdgePos)e1; e += 32) {
       const int32_t d = idx[e];
       if (d < 0 || (int64_t)d >= n) {
         atomicOr(status, kBadId);
