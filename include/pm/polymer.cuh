@@ -1533,6 +1533,7 @@ struct Engine {
     for (int i = 0; i < 3; ++i)
       if (h_cnt[i].err) {
         unsigned e = h_cnt[i].err;
+        reset_counters();  // reported here, and not by the next call again
         fail(e & kErrTimeout ? PM_ERR_TIMEOUT : PM_ERR_CUDA,
              std::string("device error word ") + std::to_string(e) +
                  (e & kErrQueueOverflow ? " (queue overflow)" : "") +

@@ -215,11 +215,13 @@ void run_cc_union_find(pm_graph *g, int32_t *d_labels, pm_traversal_stats *st) {
   PM_LAUNCH_COOP(k_uf, round_grid(E, per_sm), kRoundThreads, E.stream, E.g, d_labels, edges);
   E.prof.end(E.stream);
   if (st) {
-    const Counters *h = E.read_counters();
+    // this launch raises no error word: only its own count is read
+    PM_CUDA(cudaMemcpyAsync(&E.h_cnt->edges, edges, sizeof *edges, cudaMemcpyDeviceToHost, E.stream));
+    PM_CUDA(cudaStreamSynchronize(E.stream));
     pm_traversal_stats s{};
     s.rounds = 3;  // union-find passes over the vertices
     s.dense_rounds = 0;
-    s.edges_visited = (int64_t)h[0].edges;  // edges linked
+    s.edges_visited = (int64_t)E.h_cnt->edges;  // edges linked
     s.reached = g->n;
     *st = s;
   }
