@@ -26,7 +26,7 @@ struct BfsWork {
   uint32_t *bits[2];     // frontier of even / odd levels, valid after a dense round
   RoundQueue q[2];
   RoundCount *count;     // three slots, level % 3
-  pm_traversal_stats *stats;
+  RoundsEnd *end;
 };
 
 // One dense round: next = the unvisited vertices with an in-neighbour in cur.
@@ -121,32 +121,37 @@ __device__ __forceinline__ void bfs_pull(const GraphView &g, const BfsWork &w, c
   }
 }
 
-__global__ void __launch_bounds__(kRoundThreads, 2) k_bfs(GraphView g, BfsWork w, int32_t src,
-                                                                   int64_t threshold) {
+__global__ void __launch_bounds__(kRoundThreads, 2) k_bfs(GraphView g, BfsWork w, RoundsEnd from, int32_t src,
+                                                          int64_t threshold) {
   cg::grid_group grid = cg::this_grid();
   const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, gsize = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t v = gtid; v < g.n; v += gsize) {
-    w.parents[v] = v == src ? src : -1;
-    w.depth[v] = v == src ? 0 : -1;
+  PM_ROUND_STATS(st, gtid, from);
+  if (from.level == 1) {
+    for (int64_t v = gtid; v < g.n; v += gsize) {
+      w.parents[v] = v == src ? src : -1;
+      w.depth[v] = v == src ? 0 : -1;
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 32) round_start(g, src, w.q[0], w.count);
+    grid.sync();
   }
-  if (blockIdx.x == 0 && threadIdx.x < 32) round_start(g, src, w.q[0], w.count);
-  grid.sync();
-  pm_traversal_stats st{};
-  st.reached = 1;
-  bool have_bits = false, have_queue = true;
-  for (int32_t level = 1;; ++level) {
+  bool have_bits = from.have_bits, more = false;
+  int32_t level = from.level;
+  for (;; ++level) {
     RoundCount *cur = w.count + (level - 1) % 3, *nxt = w.count + level % 3;
     RoundCount f = round_read(cur);
     const unsigned long long fsize = f.size, fedges = f.edges;
-    if (level > 1) st.reached += (int64_t)fsize;
-    if (fsize == 0) break;
+    more = fsize != 0 && level - from.level == kRoundsPerLaunch;
+    if (fsize == 0 || more) break;
     const bool dense = (long long)(fsize + fedges) >= threshold;
     const RoundQueue &q = w.q[(level - 1) & 1], &qn = w.q[level & 1];
     uint32_t *bits = w.bits[(level - 1) & 1], *bits_next = w.bits[level & 1];
-    st.rounds++;
-    st.dense_rounds += dense;
-    st.edges_visited += (int64_t)fedges;
-    if (gtid == 0) w.count[(level + 1) % 3] = RoundCount{};
+    if (gtid == 0) {
+      st.rounds++;
+      st.dense_rounds += dense;
+      st.edges_visited += (int64_t)fedges;
+      st.reached += (int64_t)fsize;
+      w.count[(level + 1) % 3] = RoundCount{};
+    }
     unsigned long long size = 0, edges = 0;
     if (dense) {
       if (!have_bits) {
@@ -157,7 +162,7 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_bfs(GraphView g, BfsWork w
       }
       bfs_pull(g, w, bits, bits_next, level, size, edges);
     } else {
-      if (!have_queue) {
+      if (have_bits) {
         round_bits_to_queue(g, bits, q, cur);
         grid.sync();
         f = round_read(cur);
@@ -185,11 +190,10 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_bfs(GraphView g, BfsWork w
           });
     }
     have_bits = dense;
-    have_queue = !dense;
     round_count_add(size, edges, nxt);
     grid.sync();
   }
-  if (gtid == 0) *w.stats = st;
+  if (gtid == 0) *w.end = RoundsEnd{st, level, more, have_bits, 0};
 }
 
 void run_bfs_rounds(pm_graph *g, int32_t src, int32_t *d_parents, int32_t *d_depth, int64_t threshold,
@@ -206,16 +210,14 @@ void run_bfs_rounds(pm_graph *g, int32_t src, int32_t *d_parents, int32_t *d_dep
     w.q[k].pieces = pc + k * pieces;
   }
   w.count = (RoundCount *)g->scratch_buf(30, 3 * sizeof(RoundCount));
-  static_assert(sizeof(pm_traversal_stats) <= 3 * sizeof(Counters), "written to the pinned counter words");
-  w.stats = (pm_traversal_stats *)E.h_cnt;  // pinned: the kernel writes it over the bus
+  w.end = (RoundsEnd *)E.h_cnt;
   static const int per_sm = round_occupancy(k_bfs);
   E.prof.begin("bfs", E.stream);
-  PM_LAUNCH_COOP(k_bfs, round_grid(E, per_sm), kRoundThreads, E.stream, E.g, w, src, threshold);
-  E.prof.end(E.stream);
-  if (st) {
-    PM_CUDA(cudaStreamSynchronize(E.stream));
-    std::memcpy(st, w.stats, sizeof *st);
-  }
+  const pm_traversal_stats s = run_rounds(E, [&](const RoundsEnd &from) {
+    PM_LAUNCH_COOP(k_bfs, round_grid(E, per_sm), kRoundThreads, E.stream, E.g, w, from, src, threshold);
+    E.prof.end(E.stream);
+  });
+  if (st) *st = s;
 }
 
 }  // namespace pm

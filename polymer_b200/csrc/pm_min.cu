@@ -26,22 +26,24 @@ struct MinWork {
   int32_t *val, *before, *stamp;
   RoundQueue q[2];
   RoundCount *count;  // three slots, level % 3
-  pm_traversal_stats *stats;
+  RoundsEnd *end;
 };
 
 // W: val + weight from the source src (BellmanFord); otherwise every vertex
 // starts with its id and in the frontier (labels).
 template <bool W>
 __global__ void __launch_bounds__(kRoundThreads, 2) k_min_rounds(GraphView g, const int32_t *__restrict__ weight,
-                                                                 MinWork w, int32_t src, int64_t threshold) {
+                                                                 MinWork w, RoundsEnd from, int32_t src, int64_t threshold) {
   cg::grid_group grid = cg::this_grid();
   const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, gsize = (int64_t)gridDim.x * blockDim.x;
   constexpr int64_t kTile = (int64_t)kRoundThreads * kStep;
-  for (int64_t v = gtid; v < g.n; v += gsize) {
-    w.val[v] = W ? (v == src ? 0 : kDevBFInf) : (int32_t)v;
-    w.stamp[v] = 0;
-  }
-  if (W && blockIdx.x == 0 && threadIdx.x < 32) round_start(g, src, w.q[0], w.count);
+  const bool fresh = from.level == 1;
+  if (fresh)
+    for (int64_t v = gtid; v < g.n; v += gsize) {
+      w.val[v] = W ? (v == src ? 0 : kDevBFInf) : (int32_t)v;
+      w.stamp[v] = 0;
+    }
+  if (W && fresh && blockIdx.x == 0 && threadIdx.x < 32) round_start(g, src, w.q[0], w.count);
   // the vertices of the block's tiles for which in(v) holds become the frontier
   // q, counted in c
   auto collect = [&](auto &&in, const RoundQueue &q, RoundCount *c) {
@@ -65,23 +67,29 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_min_rounds(GraphView g, co
     }
     round_count_add(size, edges, c);
   };
-  if (!W) collect([](int) { return true; }, w.q[0], w.count);
+  if (!W && fresh) collect([](int) { return true; }, w.q[0], w.count);
   grid.sync();
   // a source's value as its piece or row is taken: one lowered later in the
   // round is in the next frontier and pushes again
   auto value_of = [&](int s) { return *((volatile int32_t *)w.val + s); };
-  pm_traversal_stats st{};
-  for (int32_t level = 1;; ++level) {
+  PM_ROUND_STATS(st, gtid, from);
+  int32_t level = from.level;
+  bool more = false;
+  for (;; ++level) {
     RoundCount *cur = w.count + (level - 1) % 3, *nxt = w.count + level % 3;
     const RoundCount f = round_read(cur);
     const unsigned long long fsize = f.size, fedges = f.edges;
-    if (fsize == 0 || st.rounds > (int64_t)g.n + 1) break;
+    if (fsize == 0 || level > (int64_t)g.n + 2) break;  // level - 1 rounds are done
+    more = level - from.level == kRoundsPerLaunch;
+    if (more) break;
     const bool dense = (long long)(fsize + fedges) >= threshold;
     const RoundQueue &q = w.q[(level - 1) & 1], &qn = w.q[level & 1];
-    st.rounds++;
-    st.dense_rounds += dense;
-    st.edges_visited += (int64_t)fedges;
-    if (gtid == 0) w.count[(level + 1) % 3] = RoundCount{};
+    if (gtid == 0) {
+      st.rounds++;
+      st.dense_rounds += dense;
+      st.edges_visited += (int64_t)fedges;
+      w.count[(level + 1) % 3] = RoundCount{};
+    }
     if (dense) {
       for (int64_t v0 = gtid; v0 < g.n; v0 += kStep * gsize) {  // four loads in flight
         int32_t x[kStep];
@@ -133,7 +141,7 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_min_rounds(GraphView g, co
     }
     grid.sync();
   }
-  if (gtid == 0) *w.stats = st;
+  if (gtid == 0) *w.end = RoundsEnd{st, level, more, 0, 0};
 }
 
 template <bool W>
@@ -151,15 +159,15 @@ static pm_traversal_stats run_min(pm_graph *g, const int32_t *weight, int32_t sr
     w.q[k].pieces = pc + k * pieces;
   }
   w.count = (RoundCount *)g->scratch_buf(30, 3 * sizeof(RoundCount));
-  static_assert(sizeof(pm_traversal_stats) <= 3 * sizeof(Counters), "written to the pinned counter words");
-  w.stats = (pm_traversal_stats *)E.h_cnt;  // pinned: the kernel writes it over the bus
+  w.end = (RoundsEnd *)E.h_cnt;
   if (!W) PM_CUDA(cudaMemsetAsync(w.count, 0, 3 * sizeof(RoundCount), E.stream));
   static const int per_sm = round_occupancy(k_min_rounds<W>);
   E.prof.begin(tag, E.stream);
-  PM_LAUNCH_COOP((k_min_rounds<W>), round_grid(E, per_sm), kRoundThreads, E.stream, E.g, weight, w, src, threshold);
-  E.prof.end(E.stream);
-  PM_CUDA(cudaStreamSynchronize(E.stream));
-  const pm_traversal_stats st = *w.stats;
+  const pm_traversal_stats st = run_rounds(E, [&](const RoundsEnd &from) {
+    PM_LAUNCH_COOP((k_min_rounds<W>), round_grid(E, per_sm), kRoundThreads, E.stream, E.g, weight, w, from, src,
+                   threshold);
+    E.prof.end(E.stream);
+  });
   E.prof.set_passes((int)st.rounds);
   return st;
 }

@@ -41,7 +41,7 @@ struct MsbfsWork {
   u64 *visited;
   int32_t *touched;  // vertices a sparse level reached, each once
   RoundQueue q[2];
-  RoundCount *count;   // three slots, level % 3
+  RoundCount *count;   // three slots, level % 3, and the call's sums
   unsigned *ntouched;  // three slots, level % 3
   const int32_t *order;  // rows by in-degree, longest first
   const int2 *long_pieces;  // {vertex, first in-edge of the piece} of the rows [0, rc)
@@ -49,7 +49,7 @@ struct MsbfsWork {
   const int32_t *sources;
   int k;
   int32_t *depth;
-  pm_traversal_stats *stats;
+  RoundsEnd *end;
 };
 
 // OR over the lanes of `width` consecutive lanes.
@@ -256,20 +256,22 @@ __device__ __forceinline__ void msbfs_depths(const MsbfsWork &w, int64_t n, int3
   }
 }
 
-__global__ void __launch_bounds__(kRoundThreads, 2) k_msbfs(GraphView g, MsbfsWork w, int64_t threshold) {
+__global__ void __launch_bounds__(kRoundThreads, 2) k_msbfs(GraphView g, MsbfsWork w, RoundsEnd from,
+                                                            int64_t threshold) {
   cg::grid_group grid = cg::this_grid();
   const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, gsize = (int64_t)gridDim.x * blockDim.x;
   const int64_t n = g.n;
   const u64 full = w.k == 64 ? ~0ull : (1ull << w.k) - 1ull;
   auto slot = [&](int32_t t) { return w.ring + (int64_t)(t % w.slots) * n; };
-  for (int64_t v = gtid; v < n; v += gsize) slot(0)[v] = slot(1)[v] = w.visited[v] = 0ull;
-  if (gtid < 3) {
-    w.count[gtid] = RoundCount{};
-    w.ntouched[gtid] = 0;
+  const bool fresh = from.level == 1;
+  if (fresh) {
+    for (int64_t v = gtid; v < n; v += gsize) slot(0)[v] = slot(1)[v] = w.visited[v] = 0ull;
+    if (gtid < 3) w.ntouched[gtid] = 0;
+    if (gtid < 4) w.count[gtid] = RoundCount{};
+    grid.sync();
   }
-  grid.sync();
   MsbfsSums sum;
-  if (blockIdx.x == 0 && threadIdx.x < 32) {  // the sources: a vertex may hold several
+  if (fresh && blockIdx.x == 0 && threadIdx.x < 32) {  // the sources: a vertex may hold several
     bool act[kStep] = {};
     int d[kStep] = {}, deg[kStep] = {};
     u64 size = 0, edges = 0;
@@ -297,21 +299,23 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_msbfs(GraphView g, MsbfsWo
     }
   }
   grid.sync();
-  pm_traversal_stats st{};
-  bool have_queue = true;  // and visited holds every bit so far
-  int32_t flushed = 0;  // levels below this have their depths written
-  int32_t level = 1;
+  PM_ROUND_STATS(st, gtid, from);
+  bool have_queue = !from.have_bits;  // and visited holds every bit so far
+  bool more = false;
+  int32_t flushed = from.flushed;  // levels below this have their depths written
+  int32_t level = from.level;
   for (;; ++level) {
     RoundCount *cur = w.count + (level - 1) % 3, *nxt = w.count + level % 3;
     RoundCount f = round_read(cur);
-    if (f.size == 0) break;
+    more = f.size != 0 && level - from.level == kRoundsPerLaunch;
+    if (f.size == 0 || more) break;
     const bool dense = (long long)(f.size + f.edges) >= threshold;
     const RoundQueue &q = w.q[(level - 1) & 1], &qn = w.q[level & 1];
     const u64 *front = slot(level - 1);
     u64 *next = slot(level);
-    st.rounds++;
-    st.dense_rounds += dense;
     if (gtid == 0) {
+      st.rounds++;
+      st.dense_rounds += dense;
       w.count[(level + 1) % 3] = RoundCount{};
       w.ntouched[(level + 1) % 3] = 0;
     }
@@ -395,14 +399,14 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_msbfs(GraphView g, MsbfsWo
     grid.sync();
   }
   // the last levels' depths (level - 1 held the last words)
-  msbfs_depths(w, n, flushed, level - flushed, flushed == 0);
-  RoundCount *total = w.count + level % 3;  // cleared a level ago
+  if (!more) msbfs_depths(w, n, flushed, level - flushed, flushed == 0);
+  RoundCount *total = w.count + 3;
   round_count_add(sum.reached, sum.outdeg, total);
   grid.sync();
   if (gtid == 0) {
     st.reached = (int64_t)((volatile RoundCount *)total)->size;
     st.edges_visited = (int64_t)((volatile RoundCount *)total)->edges;
-    *w.stats = st;
+    *w.end = RoundsEnd{st, level, more, !have_queue, flushed};
   }
 }
 
@@ -424,7 +428,7 @@ void run_msbfs(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_depth, i
       w.ring = (u64 *)g->scratch_buf(0, (size_t)n * 8 * w.slots);
       w.visited = (u64 *)g->scratch_buf(2, (size_t)n * 8);
       pc = (int2 *)g->scratch_buf(1, 2 * pieces * sizeof(int2));
-      w.count = (RoundCount *)g->scratch_buf(30, 3 * sizeof(RoundCount) + 16);
+      w.count = (RoundCount *)g->scratch_buf(30, 4 * sizeof(RoundCount) + 16);
       order = &ensure_row_order(g, false);
       break;
     } catch (const Failure &f) {
@@ -438,7 +442,7 @@ void run_msbfs(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_depth, i
     w.q[i].pieces = pc + i * pieces;
   }
   w.touched = E.defer;
-  w.ntouched = (unsigned *)(w.count + 3);
+  w.ntouched = (unsigned *)(w.count + 4);
   w.order = order->order.as<int32_t>();
   w.long_pieces = order->pieces.as<int2>();
   w.np = order->npieces;
@@ -448,14 +452,13 @@ void run_msbfs(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_depth, i
   w.sources = d_sources;
   w.k = k;
   w.depth = d_depth;
-  static_assert(sizeof(pm_traversal_stats) <= 3 * sizeof(Counters), "written to the pinned counter words");
-  w.stats = (pm_traversal_stats *)E.h_cnt;
+  w.end = (RoundsEnd *)E.h_cnt;
   static const int per_sm = round_occupancy(k_msbfs);
   E.prof.begin("bfs_multi", E.stream);
-  PM_LAUNCH_COOP(k_msbfs, round_grid(E, per_sm), kRoundThreads, E.stream, E.g, w, threshold);
-  E.prof.end(E.stream);
-  PM_CUDA(cudaStreamSynchronize(E.stream));
-  const pm_traversal_stats s = *w.stats;
+  const pm_traversal_stats s = run_rounds(E, [&](const RoundsEnd &from) {
+    PM_LAUNCH_COOP(k_msbfs, round_grid(E, per_sm), kRoundThreads, E.stream, E.g, w, from, threshold);
+    E.prof.end(E.stream);
+  });
   E.prof.set_passes((int)s.rounds);
   if (st) *st = s;
 }

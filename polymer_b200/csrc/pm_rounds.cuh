@@ -32,6 +32,23 @@ struct RoundCount {
   unsigned rows, pieces;           // queue lengths
 };
 
+// Rounds of one launch.  A traversal can take as many rounds as the graph has
+// vertices (a path; a negative cycle until it is given up), and a launch that
+// ran them all would hold the GPU for minutes: after this many it returns, the
+// host looks at RoundsEnd and launches it again from the queue or bitmap it
+// left.  A round takes 3 us or more, a launch and a wait about 15 us.
+constexpr int kRoundsPerLaunch = 1024;
+
+// How a launch ended, in pinned memory, and where the next one goes on.
+struct RoundsEnd {
+  pm_traversal_stats stats;
+  int32_t level;       // the next round
+  int32_t more;        // its frontier is not empty
+  int32_t have_bits;   // the frontier is held as a bitmap (else as a queue)
+  int32_t flushed;     // multi-source BFS: levels below have their depths written
+};
+static_assert(sizeof(RoundsEnd) <= 3 * sizeof(Counters), "written to the pinned counter words");
+
 // Queue room for any frontier of a graph with m edges: vertices with long
 // rows number at most m / kShortRow.
 inline size_t round_pieces(int64_t m) { return (size_t)(m / kShortRow + m / kPushChunk + 1); }
@@ -303,6 +320,26 @@ __device__ __forceinline__ void round_queue_to_bits(const RoundQueue &q, unsigne
 inline int round_grid(const Engine &E, int per_sm) {
   const int64_t want = std::max<int64_t>(E.g.n, E.g.m / 8) / kRoundThreads + 1;
   return (int)std::min<int64_t>(want, (int64_t)E.num_sms * per_sm);
+}
+// A kernel's statistics: thread 0 of the grid alone keeps and writes them (in
+// shared memory: a copy in every thread's registers costs spills).
+#define PM_ROUND_STATS(st, gtid, from)      \
+  __shared__ pm_traversal_stats st;         \
+  if ((gtid) == 0) st = (from).stats
+
+// Launches launch(from) until the traversal has ended; `from` starts at round 1.
+// The stream is idle afterwards.
+template <class Launch>
+inline pm_traversal_stats run_rounds(Engine &E, Launch &&launch) {
+  const RoundsEnd *end = (const RoundsEnd *)E.h_cnt;  // pinned: the kernels write it over the bus
+  RoundsEnd from{};
+  from.level = 1;
+  do {
+    launch(from);
+    PM_CUDA(cudaStreamSynchronize(E.stream));
+    from = *end;
+  } while (from.more);
+  return from.stats;
 }
 template <class K>
 int round_occupancy(K kernel) {
