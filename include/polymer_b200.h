@@ -514,7 +514,8 @@ PM_API pm_status pm_graph_get_tunable(pm_graph *g, int key, int64_t *value);
 #define PM_APP_CC 4
 #define PM_APP_BF 5
 typedef struct pm_tune_report {
-  int64_t trials;     /* candidate settings timed                 */
+  int64_t trials;     /* timings: the starting settings three times, then
+                         each candidate of a tunable that the route reads */
   double default_ms;  /* time of the settings the handle started with */
   double best_ms;     /* time of the settings kept                  */
 } pm_tune_report;

@@ -1,13 +1,15 @@
 // pm_tune.cu -- the autotuner behind pm_tune: coordinate descent over the
-// run-time tunables one application uses, timing each candidate on the
-// graph's own stream with CUDA events and keeping the fastest.
+// run-time tunables that the route an application takes on this handle reads,
+// timing each candidate on the graph's own stream with CUDA events and keeping
+// the fastest.  A tunable that the route does not read is not tried: its trials
+// time the same program, and noise could move it for a call that does read it.
 #include <algorithm>
 #include <cstring>
 #include <functional>
 #include <mutex>
 #include <vector>
 
-#include "pm_graph.cuh"
+#include "pm_sorted.cuh"
 
 namespace pm {
 void run_bfs(pm_graph *g, int32_t src, int32_t *d_parents, int32_t *d_depth, int64_t threshold,
@@ -145,20 +147,34 @@ int64_t get_tunable(pm_graph *g, int key) {
   return field(g->E.tune, key);
 }
 
+// A tunable and whether the route taken with the settings at hand reads it.
+struct TuneKey {
+  int key;
+  std::function<bool()> read;
+};
+
 // Adds application `app` to the tuned mix: its timed call (with inputs of
-// its own in tuner scratch slots) and the tunables it reads.
-static void add_app(pm_graph *g, int app, std::vector<std::function<void()>> &runs, std::vector<int> &keys) {
+// its own in tuner scratch slots) and the tunables its routes read.
+static void add_app(pm_graph *g, int app, std::vector<std::function<void()>> &runs, std::vector<TuneKey> &keys) {
   const int64_t n = g->n;
+  const Tunables &t = g->E.tune;
   auto slot = [&](int i, size_t bytes) { return g->scratch_buf(kSlotTune0 + i, bytes); };
-  auto add_keys = [&](std::initializer_list<int> ks) {
-    for (int k : ks)
-      if (std::find(keys.begin(), keys.end(), k) == keys.end()) keys.push_back(k);
+  auto add_keys = [&](std::initializer_list<int> ks, std::function<bool()> read) {
+    for (int k : ks) keys.push_back(TuneKey{k, read});
+  };
+  auto always = [] { return true; };
+  // the pulls in vertex order that run without the degree-sorted copy
+  auto add_pull = [&](bool weighted) {
+    add_keys({PM_TUNE_HEAVY_DEG, PM_TUNE_HEAVY_MODE, PM_TUNE_PULL_CTAS_PER_SM}, [g, weighted] {
+      SortedView v;
+      return !ensure_sorted(g, false, weighted, v);
+    });
   };
   switch (app) {
     case PM_APP_PAGERANK: {
       float *out = (float *)slot(0, (size_t)n * 4);
       runs.push_back([=] { run_pagerank<float>(g, 3, 0.85, out, nullptr); });
-      add_keys({PM_TUNE_HEAVY_DEG, PM_TUNE_HEAVY_MODE, PM_TUNE_PULL_CTAS_PER_SM});
+      add_pull(false);
       break;
     }
     case PM_APP_SPMV: {
@@ -167,10 +183,10 @@ static void add_app(pm_graph *g, int app, std::vector<std::function<void()>> &ru
       float *y = (float *)slot(2, (size_t)n * 4);
       fill_uniform(g, 0x7E57ull, 0, x, n);
       runs.push_back([=] { run_spmv(g, x, 3, y, nullptr); });
-      add_keys({PM_TUNE_HEAVY_DEG, PM_TUNE_HEAVY_MODE, PM_TUNE_PULL_CTAS_PER_SM});
+      add_pull(true);
       break;
     }
-    case PM_APP_BP: {
+    case PM_APP_BP: {  // counts in one launch: nothing to choose
       float *prior = (float *)slot(3, (size_t)n * 8);
       float *out = (float *)slot(4, (size_t)n * 8);
       fill_uniform(g, 0x7E58ull, 1, prior, 2 * n);
@@ -178,7 +194,6 @@ static void add_app(pm_graph *g, int app, std::vector<std::function<void()>> &ru
         const float psi[4] = {0.9f, 0.1f, 0.1f, 0.9f};
         run_bp(g, prior, psi, 3, out);
       });
-      add_keys({PM_TUNE_HEAVY_DEG, PM_TUNE_HEAVY_MODE, PM_TUNE_PULL_CTAS_PER_SM});
       break;
     }
     case PM_APP_BFS: {
@@ -188,14 +203,18 @@ static void add_app(pm_graph *g, int app, std::vector<std::function<void()>> &ru
       runs.push_back([=] {
         for (int32_t s : srcs) run_bfs(g, s, p, d, g->m / g->E.tune.bfs_div, nullptr);
       });
-      add_keys({PM_TUNE_BFS_DIV, PM_TUNE_CTA_EXPAND, PM_TUNE_GRID_EXPAND, PM_TUNE_HEAVY_DEG});
+      add_keys({PM_TUNE_BFS_DIV}, always);
+      add_keys({PM_TUNE_CTA_EXPAND, PM_TUNE_GRID_EXPAND}, [&t] { return !t.cuda_graphs; });
       break;
     }
     case PM_APP_CC: {
       int32_t *l = (int32_t *)slot(7, (size_t)n * 4);
       runs.push_back([=] { run_cc(g, l, g->m / g->E.tune.cc_div, nullptr); });
-      add_keys({PM_TUNE_CC_DIV, PM_TUNE_CTA_EXPAND, PM_TUNE_GRID_EXPAND, PM_TUNE_HEAVY_DEG,
-                PM_TUNE_HEAVY_MODE, PM_TUNE_PULL_CTAS_PER_SM});
+      auto rounds = [g, &t] { return !g->symmetric || t.cc_mode != 0; };  // not the union-find
+      add_keys({PM_TUNE_CC_DIV}, rounds);
+      add_keys({PM_TUNE_CTA_EXPAND, PM_TUNE_GRID_EXPAND, PM_TUNE_HEAVY_DEG, PM_TUNE_HEAVY_MODE,
+                PM_TUNE_PULL_CTAS_PER_SM},
+               [rounds, &t] { return rounds() && (t.push_agg || t.pull_stage); });
       break;
     }
     case PM_APP_BF: {
@@ -203,8 +222,11 @@ static void add_app(pm_graph *g, int app, std::vector<std::function<void()>> &ru
       const int32_t src = tune_sources(g, 1)[0];
       int32_t *d = (int32_t *)slot(8, (size_t)n * 4);
       runs.push_back([=] { run_bellman_ford(g, src, d, g->m / g->E.tune.bf_div, nullptr); });
-      add_keys({PM_TUNE_BF_DELTA, PM_TUNE_BF_DENSE, PM_TUNE_BF_DIV, PM_TUNE_CTA_EXPAND, PM_TUNE_GRID_EXPAND,
-                PM_TUNE_HEAVY_DEG, PM_TUNE_HEAVY_MODE, PM_TUNE_PULL_CTAS_PER_SM});
+      add_keys({PM_TUNE_BF_DELTA, PM_TUNE_BF_DENSE, PM_TUNE_BF_DIV}, always);
+      // the host-driven schedules: their pushes and pulls
+      add_keys({PM_TUNE_CTA_EXPAND, PM_TUNE_GRID_EXPAND, PM_TUNE_HEAVY_DEG},
+               [&t] { return t.bf_dense != 2 || t.bf_delta > 0 || t.push_agg; });
+      add_keys({PM_TUNE_HEAVY_MODE, PM_TUNE_PULL_CTAS_PER_SM}, [&t] { return t.bf_dense == 0; });
       break;
     }
     default:
@@ -216,8 +238,18 @@ void tune(pm_graph *g, const int *apps, int count, pm_tune_report *rep) {
   Engine &E = g->E;
   if (count < 1 || count > 6) fail(PM_ERR_INVALID_ARG, "application count must be in [1, 6]");
   std::vector<std::function<void()>> runs;
-  std::vector<int> keys;
+  std::vector<TuneKey> keys;
   for (int i = 0; i < count; ++i) add_app(g, apps[i], runs, keys);
+  // one entry per tunable, read when any application's route reads it
+  std::vector<TuneKey> once;
+  for (const TuneKey &k : keys) {
+    auto same = std::find_if(once.begin(), once.end(), [&](const TuneKey &o) { return o.key == k.key; });
+    if (same == once.end()) {
+      once.push_back(k);
+    } else {
+      same->read = [a = same->read, b = k.read] { return a() || b(); };
+    }
+  }
   // the objective: the summed time of the mix
   std::function<void()> run = [&runs] {
     for (auto &r : runs) r();
@@ -249,11 +281,19 @@ void tune(pm_graph *g, const int *apps, int count, pm_tune_report *rep) {
   };
   double best_ms = 0.0, default_ms = 0.0;
   try {
-    best_ms = default_ms = time_once();
+    // the starting settings three times: a setting is kept only when it beats
+    // the best of them
+    for (int i = 0; i < 3; ++i) {
+      const double ms = time_once();
+      default_ms = i ? std::min(default_ms, ms) : ms;
+    }
+    best_ms = default_ms;
     // coordinate descent; a second sweep only when the first moved something
     for (int sweep = 0; sweep < 2; ++sweep) {
     bool moved = false;
-    for (int key : keys) {
+    for (const TuneKey &k : once) {
+      if (!k.read()) continue;
+      const int key = k.key;
       std::vector<int64_t> cands;
       switch (key) {
         case PM_TUNE_HEAVY_DEG: cands = {512, 1024, 2048, 4096, 8192, 32768}; break;
