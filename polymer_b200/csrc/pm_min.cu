@@ -8,17 +8,22 @@
 // A round pushes val[s] (+ weight) over the frontier's out-edges from queues
 // whose rows are cut to bounded pieces (pm_rounds.cuh); the next frontier is
 // what fell.  Rounds below the threshold learn that from the atomics' results
-// (a stamp keeps a vertex from being queued twice).  Rounds at or above it
-// issue atomics without results, skipped when the target's value as this SM
+// (a stamp keeps a vertex from being queued twice).  BellmanFord's rounds at or
+// above it issue atomics without results, skipped when the target's value as this SM
 // last saw it is already no larger (values only fall, so one seen earlier is
 // never below the current one), and find what fell by comparing with a copy
-// taken at the round's start.
+// taken at the round's start.  Labels pull in those rounds (labels_pull).
 //
 // What bounds it: the gathers of the targets' values in the one or two rounds
 // that push most of the graph (200 G edges/s), and, on small graphs, the
 // barriers.  BellmanFord on the symmetrised 2^22-vertex, 128 M-edge R-MAT
-// (weights 1..22): 1.69 ms as a host loop -> 1.16 ms here.
+// (weights 1..22): 1.69 ms as a host loop -> 1.16 ms here.  Labels: a vertex
+// order with locality has six or seven dense rounds, in which pushes lost to the
+// host loop's pulls: 2^23 vertices, 76 M edges, most of them to near ids, 2.50 ms
+// as a host loop, 3.85 with dense rounds pushed, 1.69 pulled; a directed 2^22-vertex
+// R-MAT 1.48, 0.86 and 0.84 ms.
 #include "pm_rounds.cuh"
+#include "pm_sorted.cuh"
 
 namespace pm {
 
@@ -27,7 +32,105 @@ struct MinWork {
   RoundQueue q[2];
   RoundCount *count;  // three slots, level % 3
   RoundsEnd *end;
+  // labels: the rows by in-degree, longest first (pm_sorted.cuh)
+  const int32_t *order;
+  const int2 *long_pieces;  // {vertex, first in-edge of the piece} of the rows [0, rc)
+  int32_t np, rc, rh, rm;
 };
+
+// The least of m and the labels of in-edges e, e + width, ... below e1.
+__device__ __forceinline__ int32_t labels_least(const GraphView &g, const int32_t *val, int32_t m, EdgePos e, EdgePos e1,
+                                                int width) {
+  for (; e < e1; e += kStep * width) {
+    int s[kStep];
+    int32_t x[kStep];
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) s[u] = e + u * width < e1 ? checked_id(g, __ldg(g.in.idx + e + u * width)) : -1;
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) x[u] = s[u] >= 0 ? val[s[u]] : INT32_MAX;
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) m = min(m, x[u]);
+  }
+  return m;
+}
+
+// One dense round of label propagation: every vertex takes the least label of
+// its in-neighbours, in the frontier or not (one that is not was pushed when
+// it fell: taking it again changes nothing), and is queued when it fell.  A
+// label another warp lowers meanwhile may be read before or after: the vertex
+// that lowered it is in the next frontier.  The rows are split as the
+// multi-source BFS splits its own: pieces of the longest by a CTA each, then a
+// warp or kSubLanes lanes per row, the short ones in vertex order.
+__device__ __forceinline__ void labels_pull(const GraphView &g, const MinWork &w, int32_t level, const RoundQueue &q,
+                                            RoundCount *c, unsigned long long &size, unsigned long long &edges) {
+  const int lane = lane_id();
+  const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, gsize = (int64_t)gridDim.x * blockDim.x;
+  auto queue_one = [&](bool fell, int v) {  // by the whole warp
+    const bool act[kStep] = {fell, false, false, false};
+    const int d[kStep] = {v, 0, 0, 0};
+    const int deg[kStep] = {fell ? __ldg(g.out.off + v + 1) - __ldg(g.out.off + v) : 0, 0, 0, 0};
+    size += fell;
+    edges += (unsigned)deg[0];
+    round_append(act, d, deg, q, c);
+  };
+  for (int p = blockIdx.x; p < w.np; p += gridDim.x) {
+    const int2 pc = __ldg(w.long_pieces + p);
+    const EdgePos e1 = edge_end((EdgePos)pc.y, kOrderPiece, (EdgePos)__ldg(g.in.off + pc.x + 1));
+    int32_t m = labels_least(g, w.val, INT32_MAX, (EdgePos)pc.y + threadIdx.x, e1, kRoundThreads);
+    m = __reduce_min_sync(0xffffffffu, m);
+    bool fell = false;  // queued by the first of the row's pieces to lower it
+    if (lane == 0 && m < *((volatile int32_t *)w.val + pc.x) && m < atomicMin(w.val + pc.x, m))
+      fell = atomicExch(w.stamp + pc.x, level) != level;
+    queue_one(fell, pc.x);
+  }
+  const int64_t n1 = w.rh - w.rc, n2 = ((int64_t)(w.rm - w.rh) * kSubLanes + 31) / 32;
+  for (int64_t t = gtid >> 5; t < n1 + n2; t += gsize >> 5) {
+    const bool whole = t < n1;  // the same for the whole warp
+    const int r = whole ? w.rc + (int)t : w.rh + (int)((t - n1) * (32 / kSubLanes)) + lane / kSubLanes;
+    const int width = whole ? 32 : kSubLanes, sub = whole ? lane : lane % kSubLanes;
+    int v = 0;
+    int32_t own = 0, m = INT32_MAX;
+    if (r < (whole ? w.rh : w.rm)) {
+      v = __ldg(w.order + r);
+      own = w.val[v];
+      m = labels_least(g, w.val, own, (EdgePos)__ldg(g.in.off + v) + sub, __ldg(g.in.off + v + 1), width);
+    }
+    for (int d = width / 2; d > 0; d >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, d));
+    const bool fell = sub == 0 && m < own;
+    if (fell) w.val[v] = m;
+    queue_one(fell, v);
+  }
+  constexpr int64_t kTile = (int64_t)kRoundThreads * kStep;
+  for (int64_t base = blockIdx.x * kTile; base < g.n; base += gridDim.x * kTile) {
+    bool act[kStep];
+    int v[kStep], deg[kStep];
+    EdgePos o[kStep], o1[kStep];
+    int32_t own[kStep];
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      const int64_t x = base + u * kRoundThreads + threadIdx.x;
+      v[u] = (int)min(x, (int64_t)g.n - 1);
+      o[u] = __ldg(g.in.off + v[u]);
+      o1[u] = x < g.n ? (EdgePos)__ldg(g.in.off + v[u] + 1) : o[u];
+      own[u] = w.val[v[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      act[u] = false;
+      deg[u] = 0;
+      if (o1[u] - o[u] >= kSortShort) continue;  // above
+      const int32_t m = labels_least(g, w.val, own[u], o[u], o1[u], 1);
+      act[u] = m < own[u];
+      if (act[u]) {
+        w.val[v[u]] = m;
+        deg[u] = __ldg(g.out.off + v[u] + 1) - __ldg(g.out.off + v[u]);
+        ++size;
+        edges += (unsigned)deg[u];
+      }
+    }
+    round_append_block(act, v, deg, q, c);
+  }
+}
 
 // W: val + weight from the source src (BellmanFord); otherwise every vertex
 // starts with its id and in the frontier (labels).
@@ -90,7 +193,11 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_min_rounds(GraphView g, co
       st.edges_visited += (int64_t)fedges;
       w.count[(level + 1) % 3] = RoundCount{};
     }
-    if (dense) {
+    if (!W && dense) {
+      unsigned long long size = 0, edges = 0;
+      labels_pull(g, w, level, qn, nxt, size, edges);
+      round_count_add(size, edges, nxt);
+    } else if (dense) {
       for (int64_t v0 = gtid; v0 < g.n; v0 += kStep * gsize) {  // four loads in flight
         int32_t x[kStep];
 #pragma unroll
@@ -149,9 +256,9 @@ static pm_traversal_stats run_min(pm_graph *g, const int32_t *weight, int32_t sr
                                   const char *tag) {
   Engine &E = g->E;
   const size_t pieces = round_pieces(g->m);
-  MinWork w;
+  MinWork w{};
   w.val = d_val;
-  w.before = (int32_t *)g->scratch_buf(37, (size_t)g->n * 4);
+  if (W) w.before = (int32_t *)g->scratch_buf(37, (size_t)g->n * 4);
   w.stamp = E.defer;
   int2 *pc = (int2 *)g->scratch_buf(0, 2 * pieces * sizeof(int2));
   for (int k = 0; k < 2; ++k) {
@@ -160,6 +267,15 @@ static pm_traversal_stats run_min(pm_graph *g, const int32_t *weight, int32_t sr
   }
   w.count = (RoundCount *)g->scratch_buf(30, 3 * sizeof(RoundCount));
   w.end = (RoundsEnd *)E.h_cnt;
+  if (!W) {
+    const RowOrder &o = ensure_row_order(g, false);
+    w.order = o.order.as<int32_t>();
+    w.long_pieces = o.pieces.as<int2>();
+    w.np = o.npieces;
+    w.rc = o.cuts[0];
+    w.rh = o.cuts[1];
+    w.rm = o.cuts[2];
+  }
   if (!W) PM_CUDA(cudaMemsetAsync(w.count, 0, 3 * sizeof(RoundCount), E.stream));
   static const int per_sm = round_occupancy(k_min_rounds<W>);
   E.prof.begin(tag, E.stream);
