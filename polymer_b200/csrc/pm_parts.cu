@@ -77,12 +77,16 @@ __global__ void k_parts_order(const uint32_t *key, const int32_t *val, const int
   }
 }
 
-// Slots of a slice: 32 times its longest row (a warp per slice).
-__global__ void k_parts_slices(const int32_t *deg, int64_t slices, int64_t *len) {
+// Slots of a slice: 32 times its longest row (a warp per slice); *longest: the
+// longest of all (the word starts at zero).
+__global__ void k_parts_slices(const int32_t *deg, int64_t slices, int64_t *len, int32_t *all) {
   GRID_STRIDE(p, 32 * (slices + 1)) {
     const int64_t s = p >> 5;
     const int longest = __reduce_max_sync(0xffffffffu, s < slices ? deg[p] : 0);
-    if ((p & 31) == 0) len[s] = 32 * (int64_t)longest;
+    if ((p & 31) == 0) {
+      len[s] = 32 * (int64_t)longest;
+      if (longest > *(volatile int32_t *)all) atomicMax(all, longest);
+    }
   }
 }
 __global__ void k_parts_narrow(const int64_t *in, int64_t count, int32_t *out) {
@@ -110,9 +114,32 @@ __global__ void k_parts_fill(GraphView g, PartsView a, int64_t npos, const int32
   }
 }
 
-// The layout, or false when its slots would not fit int32 or padding would
-// more than double them (a part with one row far longer than the rest), or
-// there is no memory for it: k_pagerank_parts then runs in vertex order.
+static int part_clusters(const void *kernel);
+
+// Parts of the sorted kernel in flight at once.
+static int parts_wave(const Engine &E);
+
+// Mean edges of a part from which unions of more parts than run at once take
+// the layout, and the longest row they may have, as a part of that mean.
+constexpr int64_t kPartEdges = 131072, kPartRow = 512;
+
+// The layout, or false when these parts run faster in vertex order
+// (k_pagerank_parts), its slots would not fit int32, or there is no memory for
+// it.  Where the lines lie (times of 20 iterations, vertex order against the
+// layout):
+//  * a row far longer than the rest is one lane's work and pads its slice: 60
+//    stars of 50000 vertices 60 against 182 ms.  The layout is refused when
+//    padding more than doubles the slots (a short part's slices aside).
+//  * the sorted kernel keeps half as many parts in flight (a wave), for L1's
+//    sake.  Parts that fit one wave gain (8 Erdos-Renyi parts of 100000
+//    vertices, 6 edges each: 1160 against 806 us; 5 of 8000: 119 against 100;
+//    5 rings of 8000: 83 against 76).  Beyond a wave small parts, bound by the
+//    latency of their iterations, lose (2000 parts of 500 vertices 1976 against
+//    2719 us, 400 of 8000 1239 against 1283; 100 rings of 30000 473 against 692)
+//    and large ones gain (100 of 30000 vertices, 180000 edges: 1600 against 1142;
+//    40 rings of 100000: 1250 against 1028), unless a long row bounds them, too
+//    (100 skewed parts of 30000, rows up to 11167: 28.6 against 40.3 ms; with
+//    rows up to 218: 2113 against 1667 us).
 static bool ensure_parts_layout(pm_graph *g) {
   PartsLayout &L = g->parts_layout;
   if (g->lean) return false;
@@ -124,7 +151,8 @@ static bool ensure_parts_layout(pm_graph *g) {
   std::vector<int64_t> pbase(count + 1, 0);
   for (int p = 0; p < count; ++p) pbase[p + 1] = pbase[p] + (g->parts[p + 1] - g->parts[p] + 31) / 32 * 32;
   const int64_t npos = pbase[count], slices = npos / 32;
-  if (npos >= (1ll << 31) - 64 || count > 1 << 20) {
+  const bool waves = count > parts_wave(E);
+  if (npos >= (1ll << 31) - 64 || count > 1 << 20 || (waves && m / count < kPartEdges)) {
     L.state = -1;
     return false;
   }
@@ -152,9 +180,13 @@ static bool ensure_parts_layout(pm_graph *g) {
                 deg.as<int32_t>(), odeg.as<int32_t>(), pos.as<int32_t>());
     }
     int64_t slots = 0;
+    int32_t longest = 0;
     {
+      DevBuf all(4);
+      PM_CUDA(cudaMemsetAsync(all.p, 0, 4, st));
       DevBuf len((size_t)(slices + 1) * 8), sum((size_t)(slices + 1) * 8);
-      PM_LAUNCH(k_parts_slices, E.grid_for(32 * (slices + 1), 256, 16), 256, 0, st, deg.as<int32_t>(), slices, len.as<int64_t>());
+      PM_LAUNCH(k_parts_slices, E.grid_for(32 * (slices + 1), 256, 16), 256, 0, st, deg.as<int32_t>(), slices, len.as<int64_t>(),
+                all.as<int32_t>());
       size_t tmp = 0;
       PM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp, len.as<int64_t>(), sum.as<int64_t>(), (int)(slices + 1), st));
       DevBuf tb(std::max<size_t>(tmp, 16));
@@ -162,9 +194,10 @@ static bool ensure_parts_layout(pm_graph *g) {
       PM_LAUNCH(k_parts_narrow, E.grid_for(slices + 1, 256, 16), 256, 0, st, sum.as<int64_t>(), slices + 1,
                 soff.as<int32_t>());
       PM_CUDA(cudaMemcpyAsync(&slots, sum.as<int64_t>() + slices, 8, cudaMemcpyDeviceToHost, st));
+      PM_CUDA(cudaMemcpyAsync(&longest, all.p, 4, cudaMemcpyDeviceToHost, st));
       PM_CUDA(cudaStreamSynchronize(st));
     }
-    if (slots >= (1ll << 31) - 64 || slots > 2 * m + 64 * npos) {
+    if (slots >= (1ll << 31) - 64 || slots > 2 * m + 1024ll * count || (waves && longest > m / count / kPartRow)) {
       L.state = -1;
       return false;
     }
@@ -320,6 +353,10 @@ static int part_clusters(const void *kernel) {
   PM_CUDA(cudaOccupancyMaxActiveClusters(&r, kernel, &cfg));
   return std::max(r, 1);
 }
+static int parts_wave(const Engine &E) {
+  static const int fit = part_clusters((const void *)k_pagerank_parts_sorted);
+  return std::max(1, std::min(fit, E.num_sms * kPartCtas / kPartCluster));
+}
 
 void run_pagerank_parts(pm_graph *g, int iters, double damping, float *d_out) {
   Engine &E = g->E;
@@ -335,11 +372,8 @@ void run_pagerank_parts(pm_graph *g, int iters, double damping, float *d_out) {
                       L.odeg.as<int32_t>(), L.soff.as<int32_t>(), L.ids.as<int32_t>()};
     float *c0 = (float *)g->scratch_buf(2, (size_t)L.npos * 4);
     float *c1 = (float *)g->scratch_buf(3, (size_t)L.npos * 4);
-    static const int fit = part_clusters((const void *)k_pagerank_parts_sorted);
-    const int clusters = std::min(fit, std::max(1, E.num_sms * kPartCtas / kPartCluster));
     E.prof.begin("pagerank_parts", E.stream);
-    PM_LAUNCH(k_pagerank_parts_sorted, kPartCluster * std::max(1, std::min(clusters, count)), kPartThreads, 0,
-              E.stream, a, g->parts_order.as<int32_t>(), count, iters, (float)damping, c0, c1, d_out, E.d_cnt);
+    PM_LAUNCH(k_pagerank_parts_sorted, kPartCluster * std::min(parts_wave(E), count), kPartThreads, 0, E.stream, a, g->parts_order.as<int32_t>(), count, iters, (float)damping, c0, c1, d_out, E.d_cnt);
     E.prof.end(E.stream);
     return;
   }
