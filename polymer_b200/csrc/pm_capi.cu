@@ -581,6 +581,20 @@ pm_status pm_fill_uniform_f32(pm_graph *g, uint64_t seed, int open_interval, flo
   });
 }
 
+// Whether a traversal may write its result straight into the caller's array:
+// aligned memory of the handle's own device that shares nothing with the other
+// result.  Any other array gets a copy of a result kept in scratch.
+static bool in_place(const pm_graph *g, const void *p, size_t bytes, const void *other) {
+  const uintptr_t a = (uintptr_t)p, b = (uintptr_t)other;
+  if (a % 4 != 0 || (other && a < b + bytes && b < a + bytes)) return false;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == g->device;
+}
+
 pm_status pm_bfs(pm_graph *g, int32_t src, int32_t *parents, int32_t *depth, uint32_t mem,
                  int64_t threshold, pm_traversal_stats *stats) {
   return guard(__func__, [&] {
@@ -589,11 +603,13 @@ pm_status pm_bfs(pm_graph *g, int32_t src, int32_t *parents, int32_t *depth, uin
     need(src >= 0 && src < g->n, "source out of range");
     const size_t bytes = (size_t)g->n * 4;
     const bool dev = mem == PM_MEM_DEVICE;
-    int32_t *dp = dev && parents ? parents : (int32_t *)g->scratch_buf(kSlotOut0, bytes);
-    int32_t *dd = dev && depth ? depth : (int32_t *)g->scratch_buf(kSlotOut1, bytes);
+    const bool own_p = dev && parents && in_place(g, parents, bytes, depth);
+    const bool own_d = dev && depth && in_place(g, depth, bytes, parents);
+    int32_t *dp = own_p ? parents : (int32_t *)g->scratch_buf(kSlotOut0, bytes);
+    int32_t *dd = own_d ? depth : (int32_t *)g->scratch_buf(kSlotOut1, bytes);
     run_bfs(g, src, dp, dd, threshold < 0 ? g->m / g->E.tune.bfs_div : threshold, stats);
-    if (!dev && parents) from_device(g, parents, dp, bytes, mem);
-    if (!dev && depth) from_device(g, depth, dd, bytes, mem);
+    if (!own_p && parents) from_device(g, parents, dp, bytes, mem);
+    if (!own_d && depth) from_device(g, depth, dd, bytes, mem);
     finish(g);
   });
 }
