@@ -223,10 +223,11 @@ int run_weighted_pagerank(pm_graph *g, double damping, double tol, int max_iters
   if (ensure_sorted(g, false, true, sv)) {
     // a row without in-edges holds base from the first pass on
     const double tail = (double)(n - sv.rl);
+    auto of_tail = [&](double each) { return tail > 0 ? tail * each : 0.0; };  // each may be infinite
     float *const first = a;
     launch_fill_tail(E, sv, b, base);
     const int it = iterate_sorted(g, a, b, tol, max_iters, resid, "weighted_pagerank",
-                                  tail * fabs((double)base - (double)p0), tail * fabs((double)base), nullptr,
+                                  of_tail(fabs((double)base - (double)p0)), of_tail(fabs((double)base)), nullptr,
                                   [&](int pass, float *cur, float *nxt, double2 *aux, const int *stop) {
                                     launch_sorted_pull<true>(E, sv, WPRS_F{cur, nxt, (float)damping, base}, aux, stop);
                                     if (pass == 0) launch_fill_tail(E, sv, first, base);

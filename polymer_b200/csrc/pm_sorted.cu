@@ -296,7 +296,9 @@ __global__ void __launch_bounds__(kAuxSlots) k_fix_end(double2 *aux, double tail
   if ((t & 31) == 0) s[t >> 5] = v;
   __syncthreads();
   if (t == 0) {
-    double x = st->iters == 0 ? tail_first : 0.0, y = d_tail_norm ? *d_tail_norm : tail_norm;
+    double y = d_tail_norm ? *d_tail_norm : tail_norm;
+    // a row without edges keeps its value: no change, or inf - inf = NaN
+    double x = (st->iters == 0 ? tail_first : 0.0) + (y - y);
     for (int i = 0; i < kAuxSlots / 32; ++i) {
       x += s[i].x;
       y += s[i].y;
