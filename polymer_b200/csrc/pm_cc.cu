@@ -29,11 +29,13 @@
 // what directed and partitioned handles use.
 //
 // What bounds it: the dependent reads id -> parent -> parent of a few million
-// vertices.  Each thread therefore follows kStep vertices side by side, and
-// the compressions read parents through L1 (a stale parent is an ancestor
-// too), where most trees end.  Symmetrised 2^22-vertex, 128 M-edge R-MAT:
-// 380 us as eight kernels (init 5, sampling 97 + 42, compressions 101 + 40 +
-// 39, mode 18, rest 35) -> 213 us.
+// vertices.  Each thread therefore follows kStep vertices side by side, in the
+// links too, and the compressions read parents through L1 (a stale parent is an
+// ancestor too), where most trees end.  Symmetrised 2^22-vertex, 128 M-edge
+// R-MAT: 407 us as eight kernels, 244 in one launch whose links went one after
+// another, 180 here; the grid without 30 % of its edges 775, 1336 and 734 us
+// (with half the eight kernels' threads its links, 944 us of it, took as many
+// more steps in a row).
 #include <algorithm>
 
 #include "pm_rounds.cuh"
@@ -41,6 +43,7 @@
 namespace pm {
 
 constexpr int kModeSamples = kRoundThreads;
+constexpr int kFewEdges = 16;  // of a row that its own lane links in step 4
 
 __device__ __forceinline__ int32_t ld_parent(const int32_t *p, int32_t v) {
   return *((volatile const int32_t *)p + v);
@@ -60,11 +63,45 @@ __device__ __forceinline__ void uf_link(int32_t *parent, int32_t u, int32_t v) {
   }
 }
 
-// Steps a compression takes through L1 without storing: most trees are no
-// deeper.  Past them every thread stores its jumps and reads past L1, so that
-// all chains shorten together (pointer doubling): a path of n vertices in id
-// order takes log n steps, not n.
-constexpr int kShallow = 8;
+// The same for kStep pairs of parents (p1[u], p2[u]) side by side: their chains
+// of dependent reads overlap.  Pairs that are equal are linked already.
+__device__ __forceinline__ void uf_link_each(int32_t *parent, int32_t (&p1)[kStep], int32_t (&p2)[kStep]) {
+  for (;;) {
+    int32_t above[kStep], low[kStep];
+    bool more = false;
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      low[u] = min(p1[u], p2[u]);
+      above[u] = p1[u] != p2[u] ? ld_parent(parent, max(p1[u], p2[u])) : low[u];
+    }
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      const int32_t high = max(p1[u], p2[u]);
+      // a root is hung under low; when another thread was first, above is its choice
+      if (above[u] == high && above[u] != low[u]) {
+        above[u] = atomicCAS(parent + high, high, low[u]);
+        if (above[u] == high) above[u] = low[u];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      const bool open = above[u] != low[u];
+      p1[u] = open ? ld_parent(parent, above[u]) : low[u];
+      p2[u] = open ? ld_parent(parent, low[u]) : low[u];
+      more |= open;
+    }
+    if (!more) break;
+  }
+}
+
+// Steps a compression takes before it stores its jumps, and before it reads
+// past L1 as well: most trees are no deeper than the first.  Once every thread
+// does both, all chains shorten together (pointer doubling): a path of n
+// vertices in id order takes log n steps, not n.  With both at 8 a 2048 x 2048
+// grid takes 403 us and one without 30 % of its edges 885; with both at 2 191
+// and 784, but a symmetrised 2^21-vertex graph of mostly near neighbours 227
+// instead of 183; as they are 229, 734 and 169.
+constexpr int kPublish = 2, kPastL1 = 8;
 
 // parent[v] := root of v, for every v.  Writes only v's own entry; a reader of
 // parent[v] meanwhile sees either the old value or the root, both ancestors.
@@ -82,12 +119,8 @@ __device__ __forceinline__ void uf_compress(int32_t *parent, int64_t n) {
       for (int u = 0; u < kStep; ++u)
         if (p[u] != q[u]) {
           p[u] = q[u];
-          if (step < kShallow) {
-            q[u] = __ldca(parent + q[u]);
-          } else {  // a long chain: publish the jump, read what others published
-            if (v0 + u * gsize < n) parent[v0 + u * gsize] = p[u];
-            q[u] = ld_parent(parent, q[u]);
-          }
+          if (step >= kPublish && v0 + u * gsize < n) parent[v0 + u * gsize] = p[u];
+          q[u] = step < kPastL1 ? __ldca(parent + q[u]) : ld_parent(parent, q[u]);
           more |= p[u] != q[u];
         }
       if (!more) break;
@@ -163,17 +196,18 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_uf(GraphView g, int32_t *p
 #pragma unroll
     for (int u = 0; u < kStep; ++u) pd[u] = d[u] >= 0 ? ld_parent(parent, d[u]) : 0;
 #pragma unroll
-    for (int u = 0; u < kStep; ++u)
-      if (d[u] >= 0) {
-        ++mine;
-        if (pd[u] != pv[u]) uf_link(parent, (int32_t)(v0 + u * gsize), d[u]);
-      }
+    for (int u = 0; u < kStep; ++u) {
+      mine += d[u] >= 0;
+      if (d[u] < 0) pd[u] = pv[u];
+    }
+    uf_link_each(parent, pv, pd);
   }
   grid.sync();
   uf_compress(parent, n);
   grid.sync();
-  // 3. and 4.: a warp takes 32 * kStep vertices; each vertex outside the
-  // largest component has its neighbours linked by the whole warp
+  // 3. and 4.: a warp takes 32 * kStep vertices; a vertex outside the largest
+  // component links its neighbours itself when they are few, side by side with
+  // the lane's other vertices, else the whole warp does
   const int32_t L = uf_mode(parent, n);
   grid.sync();  // every block has chosen, from the same trees: they agree on L
   for (int64_t base = gtid - lane; base < n; base += kStep * gsize) {
@@ -185,9 +219,30 @@ __global__ void __launch_bounds__(kRoundThreads, 2) k_uf(GraphView g, int32_t *p
       o0[u] = __ldg(g.out.off + v);
       o1[u] = base + u * gsize + lane < n ? __ldg(g.out.off + v + 1) : 0;
     }
+    int32_t few = 0;  // the longest of this lane's short rows
 #pragma unroll
     for (int u = 0; u < kStep; ++u) {
-      unsigned todo = __ballot_sync(0xffffffffu, o0[u] < o1[u] && p[u] != L);
+      if (p[u] == L || o0[u] > o1[u]) o1[u] = o0[u];  // nothing to do
+      if (o1[u] - o0[u] <= kFewEdges) few = max(few, o1[u] - o0[u]);
+    }
+    for (int32_t k = 0; k < few; ++k) {
+      int32_t d[kStep], pd[kStep];
+#pragma unroll
+      for (int u = 0; u < kStep; ++u) {
+        const bool on = k < o1[u] - o0[u] && o1[u] - o0[u] <= kFewEdges;
+        d[u] = on ? checked_id(g, __ldg(g.out.idx + o0[u] + k)) : -1;
+        mine += on && k >= 2;  // the first two were counted above
+      }
+#pragma unroll
+      for (int u = 0; u < kStep; ++u) {
+        pd[u] = d[u] >= 0 ? ld_parent(parent, d[u]) : p[u];
+      }
+      uf_link_each(parent, p, pd);
+    }
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      if (o1[u] - o0[u] <= kFewEdges) o1[u] = o0[u];
+      unsigned todo = __ballot_sync(0xffffffffu, o0[u] < o1[u]);
       while (todo) {
         const int l = __ffs(todo) - 1;
         todo &= todo - 1;
