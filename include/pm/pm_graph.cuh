@@ -1,6 +1,7 @@
 // pm_graph.cuh -- the graph handle behind the C ABI.
 #pragma once
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -44,6 +45,16 @@ struct AllocScope {
   ~AllocScope() { set_alloc_ctx(saved); }
   AllocScope(const AllocScope &) = delete;
   AllocScope &operator=(const AllocScope &) = delete;
+};
+
+// While one lives, this thread's allocations are for something that only makes
+// calls faster: they do not take other handles' copies (reclaim_copies).
+struct PM_CXX_API OptionalAlloc {
+  bool saved;
+  OptionalAlloc();
+  ~OptionalAlloc();
+  OptionalAlloc(const OptionalAlloc &) = delete;
+  OptionalAlloc &operator=(const OptionalAlloc &) = delete;
 };
 
 // First base of pm_graph: its destructor runs after every member's, so the
@@ -154,6 +165,10 @@ struct pm_graph : pm::IdleFreeBase {
   pm::DevBuf parts_vbase, parts_order;
   pm::PartsLayout parts_layout;
   bool lean = false;  // the call runs again after running out of memory: no copies
+  // calls now running on the handle: its copies may be given back to others
+  // that run out of memory only while there are none (reclaim_copies)
+  std::mutex use_mu;
+  int users = 0;
   // 1D vertex partition across processes (pm_graph_create_partition): this
   // handle holds the edges whose destination lies in [part_lo, part_hi)
   // (rank r owns [part_bounds[r], part_bounds[r+1]); part_wbounds are the
@@ -196,7 +211,16 @@ namespace pm {
 // Builds every derived structure (CSC, groups, heavy chunks, workspaces)
 // once out.off / out.idx hold a validated CSR on the device.
 void finish_graph(pm_graph *g);
+// Gives the copies' memory back (and the captured loops that read them); false
+// when there was nothing to give.
 bool drop_copies(pm_graph *g);
+// The same for every handle on the device that no call is using: what an
+// allocation that failed (of a new graph, or of a call on another handle) asks
+// for before it reports that memory ran out.
+bool reclaim_copies(int device);
+// Handles that reclaim_copies looks at.
+void register_graph(pm_graph *g);
+void unregister_graph(pm_graph *g);
 // Rebuilds what depends on E.tune (heavy tables when heavy_deg changed from
 // old_heavy_deg, the views, the partials) and drops captured loops.
 void apply_tunables(pm_graph *g, int32_t old_heavy_deg);

@@ -41,6 +41,7 @@ struct Cache {
 };
 
 thread_local AllocCtx t_ctx;
+thread_local bool t_optional = false;
 
 Cache &cache() {
   static Cache *c = new Cache();  // never destroyed: blocks outlive static teardown order
@@ -101,6 +102,9 @@ std::atomic<long long> g_fail_after{-1};
 
 void set_alloc_fail_after(long long k) { g_fail_after.store(k < 1 ? -1 : k); }
 
+OptionalAlloc::OptionalAlloc() : saved(t_optional) { t_optional = true; }
+OptionalAlloc::~OptionalAlloc() { t_optional = saved; }
+
 AllocCtx alloc_ctx() { return t_ctx; }
 void set_alloc_ctx(AllocCtx c) { t_ctx = c; }
 
@@ -153,6 +157,15 @@ void *dev_alloc(size_t bytes, size_t *cap, int *device) {
   void *p = nullptr;
   cudaError_t e = cudaMalloc(&p, want);
   if (e == cudaErrorMemoryAllocation) {  // give the cache back and try once more
+    (void)cudaGetLastError();
+    {
+      std::lock_guard<std::mutex> lk(c.mu);
+      release_all(c);
+    }
+    e = cudaMalloc(&p, want);
+  }
+  // then what idle handles hold only to make their calls faster
+  if (e == cudaErrorMemoryAllocation && !t_optional && reclaim_copies(dev)) {
     (void)cudaGetLastError();
     {
       std::lock_guard<std::mutex> lk(c.mu);

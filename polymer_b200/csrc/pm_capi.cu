@@ -88,20 +88,46 @@ struct NvtxRange {
   NvtxRange &operator=(const NvtxRange &) = delete;
 };
 
-static thread_local pm_graph *t_entered = nullptr;  // the handle of this thread's call (enter)
+// The handle that a call entered (enter), in use until the call ends.  Calls
+// nest when an exchange function makes some of its own.
+struct HandleUse {
+  HandleUse *outer;
+  pm_graph *g = nullptr;
+  HandleUse();
+  ~HandleUse();
+  void leave() {
+    if (!g) return;
+    std::lock_guard<std::mutex> lk(g->use_mu);
+    --g->users;
+  }
+  void hold(pm_graph *h) {
+    leave();
+    std::lock_guard<std::mutex> lk(h->use_mu);
+    ++h->users;
+    g = h;
+  }
+  HandleUse(const HandleUse &) = delete;
+  HandleUse &operator=(const HandleUse &) = delete;
+};
+static thread_local HandleUse *t_use = nullptr;
+HandleUse::HandleUse() : outer(t_use) { t_use = this; }
+HandleUse::~HandleUse() {
+  leave();
+  t_use = outer;
+}
 
 template <class Fn>
 static pm_status guard(const char *name, Fn &&fn) {
   NvtxRange range(name);
   AllocScope scope(AllocCtx{});  // enter() names the call's stream
-  t_entered = nullptr;
+  HandleUse use;
   try {
     try {
       fn();
     } catch (const Failure &f) {
       // Out of memory: without the copies that only make calls faster there
       // may be room (every call has a form that does without them).
-      pm_graph *g = t_entered;
+      pm_graph *g = use.g;
       if (f.status != PM_ERR_OOM || !g || !drop_copies(g)) throw;
       struct Lean {
         pm_graph *g;
@@ -154,6 +180,7 @@ static pm_graph *new_graph(int device, bool symmetric) {
     PM_CUDA(cudaEventCreate(&g->ev0));
     PM_CUDA(cudaEventCreate(&g->ev1));
     PM_CUDA(cudaDeviceGetAttribute(&g->E.num_sms, cudaDevAttrMultiProcessorCount, device));
+    register_graph(g);
   } catch (...) {
     delete g;
     throw;
@@ -197,7 +224,7 @@ static void enter(pm_graph *g) {
   need(g != nullptr, "null graph handle");
   PM_CUDA(cudaSetDevice(g->device));
   set_alloc_ctx(AllocCtx{g->E.stream, false});  // this call's buffers live in this stream's order
-  t_entered = g;
+  t_use->hold(g);
 }
 
 extern "C" {

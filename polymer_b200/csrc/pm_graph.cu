@@ -644,6 +644,7 @@ void fill_uniform(pm_graph *g, uint64_t seed, int open, float *out, int64_t coun
 }  // namespace pm
 
 pm_graph::~pm_graph() {
+  pm::unregister_graph(this);
   if (E.stream) cudaStreamSynchronize(E.stream);
   E.release_graphs();
   E.release_side_stream();

@@ -157,6 +157,7 @@ static bool ensure_parts_layout(pm_graph *g) {
     return false;
   }
   try {
+    OptionalAlloc optional;
     int pbits = 1;
     while ((1ll << pbits) < count) ++pbits;  // at most 20
     DevBuf dp((size_t)(count + 1) * 8), order((size_t)npos * 4), deg((size_t)npos * 4), odeg((size_t)npos * 4),

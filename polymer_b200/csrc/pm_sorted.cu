@@ -1,5 +1,9 @@
 // pm_sorted.cu -- the degree-sorted copy of an adjacency (pm_sorted.cuh) and
 // PageRank and SpMV over it.
+#include <algorithm>
+#include <mutex>
+#include <vector>
+
 #include <cub/cub.cuh>
 
 #include "pm_sorted.cuh"
@@ -251,6 +255,7 @@ const SortedView *ensure_sorted(pm_graph *g, bool csr, bool weighted, SortedView
   SortedAdj &b = csr ? g->sorted_out : g->sorted_in;
   Engine &E = g->E;
   try {
+    OptionalAlloc optional;
     if (!b.view) build_sorted(g, csr, b);
     if (weighted && !b.w.p) {
       const DevBuf &w = csr ? g->w_f32_out : g->w_f32_in;
@@ -272,16 +277,53 @@ const SortedView *ensure_sorted(pm_graph *g, bool csr, bool weighted, SortedView
   return &view;
 }
 
-// Gives the copies' memory back (and the captured loops that read them); false
-// when there was nothing to give.
-bool drop_copies(pm_graph *g) {
-  if (!g->sorted_in.odeg.p && !g->sorted_out.odeg.p && g->parts_layout.state <= 0) return false;
-  PM_CUDA(cudaStreamSynchronize(g->E.stream));
+static bool has_copies(const pm_graph *g) {
+  return g->sorted_in.odeg.p || g->sorted_out.odeg.p || g->parts_layout.state > 0;
+}
+static void give_back(pm_graph *g) {
   g->E.release_graphs();
   g->sorted_in = SortedAdj{};
   g->sorted_out = SortedAdj{};
   if (g->parts_layout.state > 0) g->parts_layout = PartsLayout{};
+}
+
+bool drop_copies(pm_graph *g) {
+  if (!has_copies(g)) return false;
+  PM_CUDA(cudaStreamSynchronize(g->E.stream));
+  give_back(g);
   return true;
+}
+
+// Every handle of the process.  The list's lock is held while one is looked at,
+// so that none is destroyed meanwhile; a handle's own lock, so that no call
+// starts on it.
+namespace {
+std::mutex g_handles_mu;
+std::vector<pm_graph *> g_handles;
+}  // namespace
+
+void register_graph(pm_graph *g) {
+  std::lock_guard<std::mutex> lk(g_handles_mu);
+  g_handles.push_back(g);
+}
+void unregister_graph(pm_graph *g) {
+  std::lock_guard<std::mutex> lk(g_handles_mu);
+  g_handles.erase(std::remove(g_handles.begin(), g_handles.end(), g), g_handles.end());
+}
+
+bool reclaim_copies(int device) {
+  std::lock_guard<std::mutex> lk(g_handles_mu);
+  // freed with no stream named: a taker waits for the device first
+  AllocScope unknown(AllocCtx{});
+  bool any = false;
+  for (pm_graph *g : g_handles) {
+    if (g->device != device) continue;
+    std::unique_lock<std::mutex> own(g->use_mu, std::try_to_lock);
+    if (!own || g->users > 0 || !has_copies(g)) continue;
+    give_back(g);
+    any = true;
+  }
+  return any;
 }
 
 __global__ void __launch_bounds__(kAuxSlots) k_fix_end(double2 *aux, double tail_first, double tail_norm,
