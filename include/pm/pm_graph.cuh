@@ -29,6 +29,8 @@ struct AllocCtx {
 PM_CXX_API AllocCtx alloc_ctx();
 PM_CXX_API void set_alloc_ctx(AllocCtx c);
 PM_CXX_API void *dev_alloc(size_t bytes, size_t *cap, int *device);
+// Bytes that dev_alloc could hand out on the current device: free, or cached.
+size_t dev_available();
 // Tests: the k-th dev_alloc from now on fails with PM_ERR_OOM (k < 1: off).
 void set_alloc_fail_after(long long k);
 PM_CXX_API void dev_free(void *p, size_t cap, int device);
@@ -125,6 +127,9 @@ struct SortedView;
 struct SortedAdj {
   DevBuf odeg, off, ids, w, deg, pieces, pfirst, partials, done;
   int64_t slots = 0;
+  // what the device must have free before a build that found no room, or a copy
+  // that was given back, is tried again (0: try)
+  size_t need = 0;
   std::shared_ptr<SortedView> view;
 };
 
@@ -134,6 +139,7 @@ struct PartsLayout {
   DevBuf pbase, order, deg, odeg, soff, ids;
   int64_t npos = 0;
   int state = 0;  // 1 built, -1 not usable for these parts, 0 not built
+  size_t need = 0;  // as in SortedAdj
 };
 
 }  // namespace pm
@@ -218,6 +224,8 @@ bool drop_copies(pm_graph *g);
 // allocation that failed (of a new graph, or of a call on another handle) asks
 // for before it reports that memory ran out.
 bool reclaim_copies(int device);
+// Bytes that building the layout of the handle's parts takes at most.
+size_t parts_layout_bytes(const pm_graph *g);
 // Handles that reclaim_copies looks at.
 void register_graph(pm_graph *g);
 void unregister_graph(pm_graph *g);

@@ -182,6 +182,18 @@ void *dev_alloc(size_t bytes, size_t *cap, int *device) {
   return p;
 }
 
+size_t dev_available() {
+  int dev = 0;
+  PM_CUDA(cudaGetDevice(&dev));
+  size_t fr = 0, tot = 0;
+  PM_CUDA(cudaMemGetInfo(&fr, &tot));
+  Cache &c = cache();
+  std::lock_guard<std::mutex> lk(c.mu);
+  for (const Block &b : c.free)
+    if (b.device == dev) fr += b.cap;
+  return fr;
+}
+
 void dev_free(void *p, size_t cap, int dev) {
   if (!p) return;
   Cache &c = cache();

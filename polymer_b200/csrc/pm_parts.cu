@@ -123,6 +123,11 @@ static int parts_wave(const Engine &E);
 // the layout, and the longest row they may have, as a part of that mean.
 constexpr int64_t kPartEdges = 131072, kPartRow = 512;
 
+size_t parts_layout_bytes(const pm_graph *g) {
+  const size_t count = g->parts.size(), npos = (size_t)g->n + 32 * count;
+  return 4 * (2 * (size_t)g->m + 1024 * count) + 48 * npos + (4u << 20);
+}
+
 // The layout, or false when these parts run faster in vertex order
 // (k_pagerank_parts), its slots would not fit int32, or there is no memory for
 // it.  Where the lines lie (times of 20 iterations, vertex order against the
@@ -156,6 +161,7 @@ static bool ensure_parts_layout(pm_graph *g) {
     L.state = -1;
     return false;
   }
+  if (L.need > 0 && dev_available() < L.need) return false;  // as in ensure_sorted
   try {
     OptionalAlloc optional;
     int pbits = 1;
@@ -213,10 +219,12 @@ static bool ensure_parts_layout(pm_graph *g) {
     L.soff = std::move(soff);
     L.ids = std::move(ids);
     L.npos = npos;
+    L.need = 0;
     L.state = 1;
   } catch (const Failure &f) {
     if (f.status != PM_ERR_OOM) throw;
-    return false;  // not remembered: memory may be free the next time
+    L.need = parts_layout_bytes(g);
+    return false;
   }
   return true;
 }

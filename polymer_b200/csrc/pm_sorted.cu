@@ -189,6 +189,14 @@ const RowOrder &ensure_row_order(pm_graph *g, bool csr) {
   return o;
 }
 
+// Bytes that building (the missing parts of) a copy takes at most: the slots, the
+// tables, and while it is built the sort of the degrees.
+static size_t copy_bytes(const pm_graph *g, bool csr, bool built, bool weighted) {
+  const size_t slots = 4 * (size_t)(g->m + 2048), n = (size_t)g->n;
+  const bool ordered = (csr ? g->order_out : g->order_in).order.p != nullptr;
+  return (weighted ? slots : 0) + (built ? 0 : slots + (ordered ? 20 : 44) * n) + (4u << 20);
+}
+
 static void build_sorted(pm_graph *g, bool csr, SortedAdj &b) {
   Engine &E = g->E;
   cudaStream_t st = E.stream;
@@ -254,6 +262,10 @@ const SortedView *ensure_sorted(pm_graph *g, bool csr, bool weighted, SortedView
   if (g->is_part || g->lean || g->m > (1ll << 31) - 8192) return nullptr;
   SortedAdj &b = csr ? g->sorted_out : g->sorted_in;
   Engine &E = g->E;
+  const bool have = b.view && (!weighted || b.w.p);
+  // a build that found no room is not repeated (its sorts and passes, and the
+  // block cache emptied for nothing) until there is
+  if (!have && b.need > 0 && dev_available() < b.need) return nullptr;
   try {
     OptionalAlloc optional;
     if (!b.view) build_sorted(g, csr, b);
@@ -270,8 +282,10 @@ const SortedView *ensure_sorted(pm_graph *g, bool csr, bool weighted, SortedView
     }
   } catch (const Failure &f) {
     if (f.status != PM_ERR_OOM) throw;
+    b.need = copy_bytes(g, csr, b.view != nullptr, weighted);
     return nullptr;
   }
+  b.need = 0;
   view = *b.view;
   view.w = weighted ? b.w.as<float>() : nullptr;
   return &view;
@@ -282,9 +296,17 @@ static bool has_copies(const pm_graph *g) {
 }
 static void give_back(pm_graph *g) {
   g->E.release_graphs();
-  g->sorted_in = SortedAdj{};
-  g->sorted_out = SortedAdj{};
-  if (g->parts_layout.state > 0) g->parts_layout = PartsLayout{};
+  for (bool csr : {false, true}) {
+    SortedAdj &b = csr ? g->sorted_out : g->sorted_in;
+    if (!b.view) continue;
+    const bool weighted = b.w.p != nullptr;
+    b = SortedAdj{};
+    b.need = copy_bytes(g, csr, false, weighted);
+  }
+  if (g->parts_layout.state > 0) {
+    g->parts_layout = PartsLayout{};
+    g->parts_layout.need = parts_layout_bytes(g);
+  }
 }
 
 bool drop_copies(pm_graph *g) {
