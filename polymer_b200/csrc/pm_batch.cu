@@ -289,8 +289,8 @@ constexpr int kBfPiece = 512;  // in-edges of one warp's piece of a heavy row
 // Dense round, a warp per item: 512-edge pieces of the heavy rows (in-degree >
 // g.heavy_deg; they lower the row with atomicMin and OR the fallen lanes into
 // next_active, which starts at zero), then the light rows in order of
-// in-degree (order: pm_sorted.cu), a warp for each of [0, rh) and kBfSub lanes
-// for each of [rh, rl).  A light row is relaxed in full by its lanes, which
+// in-degree (order: pm_sorted.cu; null: by id), a warp for each of [0, rh) and
+// kBfSub lanes for each of [rh, rl).  A light row is relaxed in full by its lanes, which
 // write its next_active bytes.
 __global__ void __launch_bounds__(256, kBfCtas) k_bf_multi_pull(GraphView g, const int32_t *__restrict__ w_in,
                                                                 int32_t *dist, const u64 *__restrict__ active,
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(256, kBfCtas) k_bf_multi_pull(GraphView g, con
   EdgePos e0 = 0, e1 = 0;
   bool mine = r < rl;
   if (mine) {
-    v = __ldg(order + r);
+    v = order ? __ldg(order + r) : (int)r;
     e0 = __ldg(g.in.off + v);
     e1 = __ldg(g.in.off + v + 1);
     mine = e1 - e0 <= (EdgePos)g.heavy_deg;
@@ -431,8 +431,10 @@ void run_bf_multi(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_dist_
     return std::max(r, 1);
   }();
   const int64_t heavy_pieces = (int64_t)E.g.in.nchunks * (kChunkEdges / kBfPiece);
-  const RowOrder &o = ensure_row_order(g, false);
-  const int rh = o.cuts[1], rl = o.cuts[3];
+  // without memory for the order, a warp per row in vertex order
+  const RowOrder *o = find_row_order(g, false);
+  const int32_t *order = o ? o->order.as<int32_t>() : nullptr;
+  const int rh = o ? o->cuts[1] : (int)n, rl = o ? o->cuts[3] : (int)n;
   const int64_t items = heavy_pieces + rh + ((int64_t)(rl - rh) * kBfSub + 31) / 32;
   const unsigned pull_grid = (unsigned)((items + 7) / 8);
   const int32_t *w_in = g->w_i32_in.as<int32_t>(), *w_out = g->w_i32_out.as<int32_t>();
@@ -454,7 +456,7 @@ void run_bf_multi(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_dist_
     if (dense) {
       if (items > 0)
         PM_LAUNCH(k_bf_multi_pull, pull_grid, 256, 0, E.stream, E.g, w_in, dist, act, nxt, heavy_pieces,
-                  o.order.as<int32_t>(), rh, rl, k);
+                  order, rh, rl, k);
     } else {
       if (q > 0) {
         PM_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, qdeg, qoff, (int)q, E.stream));

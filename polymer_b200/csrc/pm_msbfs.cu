@@ -46,6 +46,7 @@ struct MsbfsWork {
   const int32_t *order;  // rows by in-degree, longest first
   const int2 *long_pieces;  // {vertex, first in-edge of the piece} of the rows [0, rc)
   int32_t np, rc, rh, rm;
+  EdgePos short_rows;    // rows below this length are taken in vertex order
   const int32_t *sources;
   int k;
   int32_t *depth;
@@ -187,7 +188,7 @@ __device__ __forceinline__ void msbfs_pull(const GraphView &g, const MsbfsWork &
 #pragma unroll
     for (int u = 0; u < kStep; ++u) {
       const int64_t v = v0 + u * gsize;
-      const bool mine = o1[u] > o[u] && o1[u] - o[u] < kSortShort;
+      const bool mine = o1[u] > o[u] && o1[u] - o[u] < w.short_rows;
       const u64 vis = need[u] | got[u];
       if (got[u] && mine) w.visited[v] = vis;
       need[u] = mine ? full & ~vis : 0ull;
@@ -414,7 +415,7 @@ void run_msbfs(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_depth, i
                pm_traversal_stats *st) {
   Engine &E = g->E;
   const int64_t n = g->n;
-  MsbfsWork w;
+  MsbfsWork w{};
   // About 1 GiB of ring at most, 3 slots at least (the front, the level being
   // built, and the next one, cleared ahead): what a call with little memory
   // left falls back to.
@@ -429,13 +430,13 @@ void run_msbfs(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_depth, i
       w.visited = (u64 *)g->scratch_buf(2, (size_t)n * 8);
       pc = (int2 *)g->scratch_buf(1, 2 * pieces * sizeof(int2));
       w.count = (RoundCount *)g->scratch_buf(30, 4 * sizeof(RoundCount) + 16);
-      order = &ensure_row_order(g, false);
-      break;
+      order = find_row_order(g, false);
+      if (order || w.slots == least) break;
     } catch (const Failure &f) {
       if (f.status != PM_ERR_OOM || w.slots == least) throw;
-      g->scratch[0].reset();
-      w.slots = least;
     }
+    g->scratch[0].reset();
+    w.slots = least;
   }
   for (int i = 0; i < 2; ++i) {
     w.q[i].rows = g->subset(i).queue;
@@ -443,12 +444,17 @@ void run_msbfs(pm_graph *g, const int32_t *d_sources, int k, int32_t *d_depth, i
   }
   w.touched = E.defer;
   w.ntouched = (unsigned *)(w.count + 4);
-  w.order = order->order.as<int32_t>();
-  w.long_pieces = order->pieces.as<int2>();
-  w.np = order->npieces;
-  w.rc = order->cuts[0];
-  w.rh = order->cuts[1];
-  w.rm = order->cuts[2];
+  w.np = w.rc = w.rh = w.rm = 0;
+  w.short_rows = ~0u;  // without memory for the order: every row
+  if (order) {
+    w.order = order->order.as<int32_t>();
+    w.long_pieces = order->pieces.as<int2>();
+    w.np = order->npieces;
+    w.rc = order->cuts[0];
+    w.rh = order->cuts[1];
+    w.rm = order->cuts[2];
+    w.short_rows = kSortShort;
+  }
   w.sources = d_sources;
   w.k = k;
   w.depth = d_depth;

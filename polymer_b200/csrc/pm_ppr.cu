@@ -156,7 +156,7 @@ __device__ __forceinline__ int4 ppr_seeds(const int32_t *__restrict__ seeds, int
                    j + 2 < k ? __ldg(seeds + j + 2) : -1, j + 3 < k ? __ldg(seeds + j + 3) : -1);
 }
 
-// order: vertices by in-degree; [0, rh) have kSortLong in-edges or more and
+// order: vertices by in-degree (null: by id); [0, rh) have kSortLong in-edges or more and
 // take a warp each, [rh, rl) a group of lanes each.
 template <int COLS>
 __global__ void __launch_bounds__(256, COLS == 32 ? 8 : 6) k_ppr_pull(GraphView g, const int32_t *__restrict__ order, int rh, int rl,
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(256, COLS == 32 ? 8 : 6) k_ppr_pull(GraphView 
   const int64_t t = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int4 seed = ppr_seeds<COLS>(seeds, k_out);
   if (t < rh) {
-    const int v = __ldg(order + t);
+    const int v = order ? __ldg(order + t) : (int)t;
     const int o = __ldg(g.in.off + v), o1 = __ldg(g.in.off + v + 1);
     Quad acc{0, 0};
     if (o1 - o > g.heavy_deg) {
@@ -466,9 +466,10 @@ static void run_ppr_cols(pm_graph *g, const int32_t *d_seeds, int k, int iters, 
   if (run_ppr_sorted<COLS>(g, d_seeds, k, iters, damping, d_out)) return;
   Engine &E = g->E;
   const int64_t n = g->n;
-  const RowOrder &o = ensure_row_order(g, false);
-  const int32_t *order = o.order.as<int32_t>();
-  const int rh = o.cuts[1], rl = o.cuts[3];
+  // without memory for the order, a warp per row in vertex order
+  const RowOrder *o = find_row_order(g, false);
+  const int32_t *order = o ? o->order.as<int32_t>() : nullptr;
+  const int rh = o ? o->cuts[1] : (int)n, rl = o ? o->cuts[3] : (int)n;
   // row n of both holds zeros (ppr_sum)
   float *c0 = (float *)g->scratch_buf(0, (size_t)(n + 1) * COLS * 4);
   float *c1 = (float *)g->scratch_buf(1, (size_t)(n + 1) * COLS * 4);
@@ -482,7 +483,7 @@ static void run_ppr_cols(pm_graph *g, const int32_t *d_seeds, int k, int iters, 
     PM_LAUNCH((k_ppr_tail<COLS>), E.grid_for((n - rl) * (COLS / 4), 256, 8), 256, 0, E.stream, E.g, order, rl, c1,
               d_out, k, d_seeds, dmp);
   const int64_t warps = rh + ((int64_t)(rl - rh) * (COLS / 4) + 31) / 32;
-  E.run_loop(loop_key("ppr", iters, k, damping, c0, c1, part, (const void *)d_seeds, d_out), [&] {
+  E.run_loop(loop_key("ppr", iters, k, damping, c0, c1, part, (const void *)d_seeds, d_out, (const void *)order), [&] {
     float *a = c0, *b = c1;
     for (int it = 0; it < iters; ++it) {
       E.prof.begin("ppr", E.stream);

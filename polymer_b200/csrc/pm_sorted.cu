@@ -189,6 +189,15 @@ const RowOrder &ensure_row_order(pm_graph *g, bool csr) {
   return o;
 }
 
+const RowOrder *find_row_order(pm_graph *g, bool csr) {
+  try {
+    return &ensure_row_order(g, csr);
+  } catch (const Failure &f) {
+    if (f.status != PM_ERR_OOM) throw;
+    return nullptr;
+  }
+}
+
 // Bytes that building (the missing parts of) a copy takes at most: the slots, the
 // tables, and while it is built the sort of the degrees.
 static size_t copy_bytes(const pm_graph *g, bool csr, bool built, bool weighted) {

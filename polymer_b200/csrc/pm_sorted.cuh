@@ -214,6 +214,9 @@ const SortedView *ensure_sorted(pm_graph *g, bool csr, bool weighted, SortedView
 
 // The rows of g's in-adjacency (or out-adjacency when csr) by degree.
 const RowOrder &ensure_row_order(pm_graph *g, bool csr);
+// The same, or null when there is no memory for it: the caller then takes the
+// rows in vertex order.
+const RowOrder *find_row_order(pm_graph *g, bool csr);
 
 // y[p] = x[order[p]]: a vector in position order.
 template <class T>
