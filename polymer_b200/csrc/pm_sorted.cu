@@ -329,25 +329,32 @@ bool drop_copies(pm_graph *g) {
 // so that none is destroyed meanwhile; a handle's own lock, so that no call
 // starts on it.
 namespace {
-std::mutex g_handles_mu;
-std::vector<pm_graph *> g_handles;
+struct Handles {
+  std::mutex mu;
+  std::vector<pm_graph *> list;
+};
+Handles &handles() {
+  static Handles *h = new Handles();  // never destroyed: handles may outlive static teardown order
+  return *h;
+}
 }  // namespace
 
 void register_graph(pm_graph *g) {
-  std::lock_guard<std::mutex> lk(g_handles_mu);
-  g_handles.push_back(g);
+  std::lock_guard<std::mutex> lk(handles().mu);
+  handles().list.push_back(g);
 }
 void unregister_graph(pm_graph *g) {
-  std::lock_guard<std::mutex> lk(g_handles_mu);
-  g_handles.erase(std::remove(g_handles.begin(), g_handles.end(), g), g_handles.end());
+  Handles &h = handles();
+  std::lock_guard<std::mutex> lk(h.mu);
+  h.list.erase(std::remove(h.list.begin(), h.list.end(), g), h.list.end());
 }
 
 bool reclaim_copies(int device) {
-  std::lock_guard<std::mutex> lk(g_handles_mu);
+  std::lock_guard<std::mutex> lk(handles().mu);
   // freed with no stream named: a taker waits for the device first
   AllocScope unknown(AllocCtx{});
   bool any = false;
-  for (pm_graph *g : g_handles) {
+  for (pm_graph *g : handles().list) {
     if (g->device != device) continue;
     std::unique_lock<std::mutex> own(g->use_mu, std::try_to_lock);
     if (!own || g->users > 0 || !has_copies(g)) continue;
