@@ -15,7 +15,10 @@
  * device.  Calls are synchronous: on return every output has been written.
  * A graph handle owns its device copy of the graph (CSR + CSC, int32 ids and
  * offsets), its frontier workspaces and a CUDA stream; distinct handles may
- * be used from distinct host threads.
+ * be used from distinct host threads.  It also keeps copies that only make its
+ * calls faster (4m + 16n bytes per direction, 4m more with weights); when
+ * memory runs out these go back, its own and those of handles that no call is
+ * using, before a call fails with PM_ERR_OOM.
  */
 #ifndef POLYMER_B200_H
 #define POLYMER_B200_H

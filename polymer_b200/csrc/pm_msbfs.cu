@@ -21,9 +21,9 @@
 // What bounds it: the first dense level, which has to look at most edges (an
 // 8-byte gather each), and the k x n depths (1 GB for 64 sources at 2^22
 // vertices).  64 sources, symmetrised 2^22-vertex, 128 M-edge R-MAT: 2.80 to
-// 3.23 ms as host-driven rounds of whole-row pulls -> 1.85 ms (the first dense
-// level 0.6 ms, 214 G gathers/s; the depths 0.2 ms).  Two CTAs per SM: three
-// (40 registers, with spills) take 1.81 ms there, but 0.85 instead of 0.80 ms
+// 3.23 ms as host-driven rounds of whole-row pulls -> 1.9 to 2.1 ms (the first
+// dense level 0.6 ms, 214 G gathers/s; the depths 0.2 ms).  Two CTAs per SM:
+// three (40 registers, with spills) take 2 % less there, but 0.85 instead of 0.80 ms
 // on a directed 2^21-vertex graph and 0.36 instead of 0.30 on 0.3 M vertices,
 // where the barriers count.
 #include "pm_rounds.cuh"

@@ -14,12 +14,12 @@
 // (nearly) the same length and one id load covers 32 edges of them.  Rows
 // without in-edges never change after the first iteration.
 //
-// What bounds it: the row gathers -- of 34 GB a pass 12 GB come from DRAM, the
+// What bounds it: the row gathers -- of 34 GB a pass 12.5 GB come from DRAM, the
 // rest from the L2 and L1 -- and the number of warps to wait for them.
 // Directed 2^24-vertex, 263 M-edge R-MAT, 32 seeds, 20 iterations: 108 ms with
 // a warp per row in vertex order and a lane per column, 73.9 ms with rows by
 // degree but the matrices in vertex order (k_ppr_pull; 72.1 with packed
-// additions and no test per gather), 64.9 ms here; 16 seeds 54.9 -> 42.9 ms,
+// additions and no test per gather), 65 to 68 ms here; 16 seeds 54.9 -> 42.9 ms,
 // 8 seeds 40.3 -> 28.9 ms.
 #include "pm_sorted.cuh"
 
