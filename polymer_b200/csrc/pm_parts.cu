@@ -15,6 +15,10 @@
 // and L2).  In vertex order a warp ran as long as its longest row -- twice the
 // mean of a random graph -- and each lane read its own ids: 256 Erdos-Renyi
 // parts, 5.1 M vertices, 41 M edges, 20 iterations: 4.13 ms -> 2.71 ms.
+#include <algorithm>
+#include <functional>
+#include <queue>
+
 #include <cooperative_groups.h>
 
 #include <cub/cub.cuh>
@@ -114,37 +118,84 @@ __global__ void k_parts_fill(GraphView g, PartsView a, int64_t npos, const int32
   }
 }
 
-static int part_clusters(const void *kernel);
+// Parts in flight at once: clusters of the sorted and of the vertex-order kernel.
+static int parts_wave(const Engine &E, bool sorted);
 
-// Parts of the sorted kernel in flight at once.
-static int parts_wave(const Engine &E);
+// The layout keeps half as many parts in flight, for L1's sake, and takes less
+// time for each; which form ends a union first depends on how many parts there
+// are, how large and how unlike.  The time of an iteration on a part of n
+// vertices and e edges, in us: what a cluster takes whatever the part (barrier,
+// launch of the loads), per edge (more when the device is full of parts), per
+// vertex, and per edge of the longest row, which is one lane's.  Fitted to 124
+// unions of 1 to 10000 parts of 50 to 100000 vertices (rings, Erdos-Renyi, in-
+// degrees skewed mildly and strongly, sizes alike and up to a factor of 20
+// apart); the form it picks is at most 9 % slower than the other one on any of
+// them, and the choice is worth up to a factor of two either way (in us, vertex
+// order against the layout: 73 parts of 4000 to 64000 vertices 736 / 361, 48 of
+// 500 to 7000 141 / 113, 8 of 100000 1160 / 806, 5 rings of 8000 83 / 76; 2000
+// of 500 1976 / 2719, 400 rings of 100 271 / 409, 133 of 860 to 1700 147 / 189).
+struct PartCost {
+  double part, edge, full, vertex, longest;
+};
+constexpr PartCost kVertexOrder{1.5, 4.2e-5, 1.1e-4, 1.6e-4, 0.042};
+constexpr PartCost kByPosition{1.3, 2.3e-5, 2.3e-5, 1.6e-4, 0.032};
 
-// Mean edges of a part from which unions of more parts than run at once take
-// the layout, and the longest row they may have, as a part of that mean.
+// The time of an iteration over all parts, sizes largest first, `wave` at once,
+// each taken as the kernels take it: by the first cluster that is free.
+static double parts_time(const PartCost &c, const std::vector<int64_t> &sizes, double edges_per_vertex, int longest,
+                         int wave) {
+  const double full = c.full * std::min(1.0, (double)sizes.size() / wave);
+  std::priority_queue<double, std::vector<double>, std::greater<double>> ends;  // of each cluster's parts so far
+  double rest = 0.0;  // small parts past the first few thousand level the clusters out
+  for (size_t i = 0; i < sizes.size(); ++i) {
+    const double n = (double)sizes[i], t = c.part + (c.edge + full) * edges_per_vertex * n + c.vertex * n + c.longest * longest;
+    if ((int)ends.size() < wave) {
+      ends.push(t);
+    } else if (i < 4096) {
+      const double first = ends.top();
+      ends.pop();
+      ends.push(first + t);
+    } else {
+      rest += t;
+    }
+  }
+  double last = 0.0;
+  for (; !ends.empty(); ends.pop()) last = ends.top();
+  return last + rest / wave;
+}
+
+// Large parts without a long row always gain: from kPartEdges edges on average,
+// no row above a kPartRow-th of that (100 Erdos-Renyi parts of 30000 vertices,
+// 180000 edges, 1600 / 1142; with rows up to 218 2113 / 1667).
 constexpr int64_t kPartEdges = 131072, kPartRow = 512;
+
+static bool parts_layout_pays(const pm_graph *g, int longest) {
+  const int64_t count = (int64_t)g->parts.size() - 1, mean = g->m / count;
+  if (mean >= kPartEdges && longest <= mean / kPartRow) return true;
+  std::vector<int64_t> sizes(count);
+  for (int64_t p = 0; p < count; ++p) sizes[p] = g->parts[p + 1] - g->parts[p];
+  std::sort(sizes.begin(), sizes.end(), std::greater<int64_t>());
+  const double epv = (double)g->m / (double)g->n;
+  return parts_time(kByPosition, sizes, epv, longest, parts_wave(g->E, true)) <=
+         parts_time(kVertexOrder, sizes, epv, longest, parts_wave(g->E, false));
+}
 
 size_t parts_layout_bytes(const pm_graph *g) {
   const size_t count = g->parts.size(), npos = (size_t)g->n + 32 * count;
-  return 4 * (2 * (size_t)g->m + 1024 * count) + 48 * npos + (4u << 20);
+  // a row's padding is at most its own length in each of the slice's 31 others
+  return 4 * ((size_t)g->m + 32 * npos) + 48 * npos + (4u << 20);
 }
 
+// Slots of the layout per edge, beside a short part's slices: a row far longer
+// than the rest of its slice reads ids that share no line with another row's
+// (60 stars of 50000 vertices 60 ms in vertex order, 182 in slots; parts whose
+// slots come to up to seven times their edges are faster all the same while they
+// are few: 5 of 8000 vertices with rows up to 3849 2977 / 2426 us).
+constexpr int kPartPadding = 8;
+
 // The layout, or false when these parts run faster in vertex order
-// (k_pagerank_parts), its slots would not fit int32, or there is no memory for
-// it.  Where the lines lie (times of 20 iterations, vertex order against the
-// layout):
-//  * a row far longer than the rest is one lane's work and pads its slice: 60
-//    stars of 50000 vertices 60 against 182 ms.  The layout is refused when
-//    padding more than doubles the slots (a short part's slices aside).
-//  * the sorted kernel keeps half as many parts in flight (a wave), for L1's
-//    sake.  Parts that fit one wave gain (8 Erdos-Renyi parts of 100000
-//    vertices, 6 edges each: 1160 against 806 us; 5 of 8000: 119 against 100;
-//    5 rings of 8000: 83 against 76).  Beyond a wave small parts, bound by the
-//    latency of their iterations, lose (2000 parts of 500 vertices 1976 against
-//    2719 us, 400 of 8000 1239 against 1283; 100 rings of 30000 473 against 692)
-//    and large ones gain (100 of 30000 vertices, 180000 edges: 1600 against 1142;
-//    40 rings of 100000: 1250 against 1028), unless a long row bounds them, too
-//    (100 skewed parts of 30000, rows up to 11167: 28.6 against 40.3 ms; with
-//    rows up to 218: 2113 against 1667 us).
+// (k_pagerank_parts), its slots would not fit int32 or be mostly padding, or
+// there is no memory for it.
 static bool ensure_parts_layout(pm_graph *g) {
   PartsLayout &L = g->parts_layout;
   if (g->lean) return false;
@@ -156,8 +207,8 @@ static bool ensure_parts_layout(pm_graph *g) {
   std::vector<int64_t> pbase(count + 1, 0);
   for (int p = 0; p < count; ++p) pbase[p + 1] = pbase[p] + (g->parts[p + 1] - g->parts[p] + 31) / 32 * 32;
   const int64_t npos = pbase[count], slices = npos / 32;
-  const bool waves = count > parts_wave(E);
-  if (npos >= (1ll << 31) - 64 || count > 1 << 20 || (waves && m / count < kPartEdges)) {
+  // without the longest row, which is known once the rows are sorted
+  if (npos >= (1ll << 31) - 64 || count > 1 << 20 || !parts_layout_pays(g, 0)) {
     L.state = -1;
     return false;
   }
@@ -204,7 +255,7 @@ static bool ensure_parts_layout(pm_graph *g) {
       PM_CUDA(cudaMemcpyAsync(&longest, all.p, 4, cudaMemcpyDeviceToHost, st));
       PM_CUDA(cudaStreamSynchronize(st));
     }
-    if (slots >= (1ll << 31) - 64 || slots > 2 * m + 1024ll * count || (waves && longest > m / count / kPartRow)) {
+    if (slots >= (1ll << 31) - 64 || slots > kPartPadding * m + 1024ll * count || !parts_layout_pays(g, longest)) {
       L.state = -1;
       return false;
     }
@@ -362,9 +413,10 @@ static int part_clusters(const void *kernel) {
   PM_CUDA(cudaOccupancyMaxActiveClusters(&r, kernel, &cfg));
   return std::max(r, 1);
 }
-static int parts_wave(const Engine &E) {
-  static const int fit = part_clusters((const void *)k_pagerank_parts_sorted);
-  return std::max(1, std::min(fit, E.num_sms * kPartCtas / kPartCluster));
+static int parts_wave(const Engine &E, bool sorted) {
+  static const int fit_sorted = part_clusters((const void *)k_pagerank_parts_sorted);
+  static const int fit_vertex = part_clusters((const void *)k_pagerank_parts);
+  return sorted ? std::max(1, std::min(fit_sorted, E.num_sms * kPartCtas / kPartCluster)) : fit_vertex;
 }
 
 void run_pagerank_parts(pm_graph *g, int iters, double damping, float *d_out) {
@@ -382,7 +434,7 @@ void run_pagerank_parts(pm_graph *g, int iters, double damping, float *d_out) {
     float *c0 = (float *)g->scratch_buf(2, (size_t)L.npos * 4);
     float *c1 = (float *)g->scratch_buf(3, (size_t)L.npos * 4);
     E.prof.begin("pagerank_parts", E.stream);
-    PM_LAUNCH(k_pagerank_parts_sorted, kPartCluster * std::min(parts_wave(E), count), kPartThreads, 0, E.stream, a, g->parts_order.as<int32_t>(), count, iters, (float)damping, c0, c1, d_out, E.d_cnt);
+    PM_LAUNCH(k_pagerank_parts_sorted, kPartCluster * std::min(parts_wave(E, true), count), kPartThreads, 0, E.stream, a, g->parts_order.as<int32_t>(), count, iters, (float)damping, c0, c1, d_out, E.d_cnt);
     E.prof.end(E.stream);
     return;
   }
@@ -390,9 +442,8 @@ void run_pagerank_parts(pm_graph *g, int iters, double damping, float *d_out) {
   float *pn = (float *)g->scratch_buf(1, (size_t)n * 4);
   float *c0 = (float *)g->scratch_buf(2, (size_t)n * 4);
   float *c1 = (float *)g->scratch_buf(3, (size_t)n * 4);
-  static const int clusters = part_clusters((const void *)k_pagerank_parts);
   E.prof.begin("pagerank_parts", E.stream);
-  PM_LAUNCH(k_pagerank_parts, kPartCluster * std::max(1, std::min(clusters, count)), kPartThreads, 0, E.stream, E.g,
+  PM_LAUNCH(k_pagerank_parts, kPartCluster * std::min(parts_wave(E, false), count), kPartThreads, 0, E.stream, E.g,
             g->parts_vbase.as<int64_t>(), g->parts_order.as<int32_t>(), count, iters, (float)damping, pc, pn, c0, c1,
             d_out, E.d_cnt);
   E.prof.end(E.stream);

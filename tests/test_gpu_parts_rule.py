@@ -1,6 +1,6 @@
 """GPU tests of which form of PageRank on parts a union takes: the layout by
 position where it is faster, vertex order for rows far longer than the rest and
-for more small parts than run at once.  The launches of the first call after the
+for many more small parts than run at once.  The launches of the first call after the
 parts were set show which (building the layout takes kernels of its own)."""
 import numpy as np
 import pytest
@@ -10,7 +10,7 @@ from test_gpu_parts_layout import _random, _star, _union
 pytestmark = pytest.mark.gpu
 
 FEW, MANY = 24, 60  # parts below and above the number that run at once (32 to 37)
-EDGES = 131072   # mean edges of a part from which longer unions take the layout
+EDGES = 131072   # mean edges of a part from which every union takes the layout
 BUILD = 4        # kernels before the size of the layout is known
 FILL = 1         # and the one that fills it
 
@@ -25,8 +25,9 @@ def _rows(longest):
 @pytest.mark.parametrize("kind,sizes,build", [
     (_random, [500] * FEW, BUILD + FILL),
     (_random, [500] * MANY, 0),                           # a second wave of small parts
-    (_star, [4097, 3], BUILD),                            # padding more than doubles the slots
-    (_star, [33, 20, 10], BUILD + FILL),                  # ... by less than a short part's slices
+    (_random, np.geomspace(318, 6360, 50).astype(int), BUILD + FILL),  # the few large ones decide
+    (_star, [4097, 3], BUILD),                            # slots that are mostly padding
+    (_star, [33, 20, 10], BUILD + FILL),                  # ... but no more than a short part's slices
     (_rows(100), [EDGES // 8 + 500] * MANY, BUILD + FILL),  # waves of large parts
     (_rows(2000), [EDGES // 8 + 500] * MANY, BUILD),        # with a long row each
 ])
